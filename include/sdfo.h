@@ -276,7 +276,8 @@ typedef struct
                                    (3) */
     int32_t triangle_cull;      /* reference-order tree: 1 = a conservative FP32
                                    triangle-box test skips closest-point tests that
-                                   cannot replace the best (same results), 2 = off;
+                                   cannot replace the best, and the fills search
+                                   warp-wide with it (same results), 2 = off;
                                    0 = default (1) */
     int32_t sparse_pair_records; /* sparse FP32 grids with 8^3 bricks created from
                                     now on keep a 32-byte record {voxel, +x

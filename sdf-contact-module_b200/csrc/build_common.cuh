@@ -1663,6 +1663,7 @@ struct DeviceRefTree
     int n = 0;
     int nnodes = 0;
     double extent = 1.0;
+    double lo[3] = {0.0, 0.0, 0.0}, hi[3] = {0.0, 0.0, 0.0}; // the root's box
     RefTreeView view() const
     {
         RefTreeView v{};
@@ -1807,6 +1808,11 @@ void build_ref_tree(DeviceRefTree& t, const double* verts, int64_t nv, const int
     });
     t.n = (int)nt;
     t.nnodes = (int)nnodes;
+    for (int a = 0; a < 3; ++a)
+    {
+        t.lo[a] = h.nodes[0].lo[a];
+        t.hi[a] = h.nodes[0].hi[a];
+    }
     t.nodes.reset(nnodes);
     t.tri9.reset(9 * n);
     t.tri_id.reset(n);
