@@ -26,6 +26,16 @@
 // and stays L1/L2-resident; the grid gather and interpolation are FP32; the
 // per-point force law of active points, the Jacobian and the reductions
 // (warp shuffles, then shared memory) are FP64.
+//
+// Most points of most poses are clear of the surface, where the law gives
+// exactly nothing.  Dense grids keep one bit per cell that says whether the
+// interpolated gap can be <= 0 there (GridView::touch); a first pass places
+// every point in FP32 and lists those whose cell has the bit, or whose cell
+// FP32 cannot tell (TouchFrame), and only the listed points take the FP64
+// transform, the gather and the law, shared out over all warps.  4096 poses of
+// a 7,680-point ring about a block's face, a quarter of them in contact: forces
+// and Jacobian 747 -> 299 us (one B200); bound by the latency of the few FP64
+// steps of a pose, no longer by the 31 M gathers.
 #include <climits>
 
 #include "interp.cuh"
@@ -33,12 +43,17 @@
 namespace sdfo {
 namespace {
 
+// Threads per pose: kContactThreads, or kFewThreads when every pose has an SM to
+// itself (fewer poses than SMs, touch bits): 33 poses of 7,680 points, forces
+// and then the measure, 78 us with 256 threads, 49 with 512 (4,096 poses with the
+// Jacobian: 299 us against 388).
 constexpr int kContactThreads = 256;
-// Jacobian pass: the points of a span of kJacSpan points that are in contact
-// are listed per warp (a warp meets at most kJacSpan / 8 of them), then all
-// warps share the span's list.
+constexpr int kFewThreads = 512;
+// Points are listed by spans of kJacSpan, per warp (a warp meets at most its
+// share of a span); then all warps share the span's list.
 constexpr int kJacSpan = 4096;
-constexpr int kJacPerWarp = kJacSpan / (kContactThreads / 32);
+// Points per thread in flight in the pass over the touch bits.
+constexpr int kAhead = 4;
 
 struct v3
 {
@@ -48,20 +63,30 @@ __device__ __forceinline__ v3 V(double x, double y, double z) { return {x, y, z}
 __device__ __forceinline__ v3 operator+(v3 a, v3 b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
 __device__ __forceinline__ v3 operator-(v3 a, v3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
 __device__ __forceinline__ v3 operator*(double s, v3 a) { return {s * a.x, s * a.y, s * a.z}; }
-__device__ __forceinline__ double dot(v3 a, v3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+// Products and sums are fused explicitly: the forward and the Jacobian kernels
+// inline the same law, and left to the compiler its contraction differs between
+// them in the last bit.
+__device__ __forceinline__ double dot(v3 a, v3 b) { return fma(a.x, b.x, fma(a.y, b.y, __dmul_rn(a.z, b.z))); }
 __device__ __forceinline__ v3 cross(v3 a, v3 b)
 {
-    return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
+    return {fma(a.y, b.z, -__dmul_rn(a.z, b.y)), fma(a.z, b.x, -__dmul_rn(a.x, b.z)),
+            fma(a.x, b.y, -__dmul_rn(a.y, b.x))};
+}
+__device__ __forceinline__ v3 add_scaled(v3 a, double s, v3 b) // a + s b
+{
+    return {fma(s, b.x, a.x), fma(s, b.y, a.y), fma(s, b.z, a.z)};
+}
+__device__ __forceinline__ v3 scaled(double s, v3 a)
+{
+    return {__dmul_rn(s, a.x), __dmul_rn(s, a.y), __dmul_rn(s, a.z)};
 }
 __device__ __forceinline__ v3 mul(const double R[9], v3 a)
 {
-    return {R[0] * a.x + R[1] * a.y + R[2] * a.z, R[3] * a.x + R[4] * a.y + R[5] * a.z,
-            R[6] * a.x + R[7] * a.y + R[8] * a.z};
+    return {dot(V(R[0], R[1], R[2]), a), dot(V(R[3], R[4], R[5]), a), dot(V(R[6], R[7], R[8]), a)};
 }
 __device__ __forceinline__ v3 mulT(const double R[9], v3 a)
 {
-    return {R[0] * a.x + R[3] * a.y + R[6] * a.z, R[1] * a.x + R[4] * a.y + R[7] * a.z,
-            R[2] * a.x + R[5] * a.y + R[8] * a.z};
+    return {dot(V(R[0], R[3], R[6]), a), dot(V(R[1], R[4], R[7]), a), dot(V(R[2], R[5], R[8]), a)};
 }
 
 template <int MODE, bool SPARSE, int BD, bool JAC>
@@ -172,25 +197,93 @@ __device__ __forceinline__ int point_state(const GridView& g, const float* __res
     const v3 xw = f.rA + st.off;
     st.rg = mul(sB.R, st.gl);
     st.gn = sqrt(dot(st.gl, st.gl));
-    st.fq = st.p * st.rg;
+    st.fq = scaled(st.p, st.rg);
     const v3 uA = f.vA + cross(f.wA, st.off);
     const v3 uB = f.vB + cross(f.wB, xw - f.rB);
     st.u = uA - uB;
     st.damp = prm.damping > 0.0 && gap < 0.0;
     st.vn = dot(st.u, st.rg);
-    if (st.damp) st.fq = st.fq + (prm.damping * (-st.vn)) * st.rg;
+    if (st.damp) st.fq = add_scaled(st.fq, prm.damping * (-st.vn), st.rg);
     const double gsafe = st.gn > 1e-30 ? st.gn : 1e-30;
-    st.un = (1.0 / gsafe) * st.rg;
+    st.un = scaled(1.0 / gsafe, st.rg);
     st.udn = dot(st.u, st.un);
-    st.ut = st.u - st.udn * st.un;
-    st.den = sqrt(dot(st.ut, st.ut) + prm.regularizer * prm.regularizer);
+    st.ut = add_scaled(st.u, -st.udn, st.un);
+    st.den = sqrt(fma(prm.regularizer, prm.regularizer, dot(st.ut, st.ut)));
     st.phat = st.p * st.gn;
     st.fric = prm.friction * st.phat > 0.0;
-    if (st.fric) st.fq = st.fq + (-prm.friction * st.phat / st.den) * st.ut;
+    if (st.fric) st.fq = add_scaled(st.fq, -prm.friction * st.phat / st.den, st.ut);
     st.dgdd = -prm.stiffness * (prm.order == 2.0 ? 2.0 * delta
                                 : prm.order == 1.0 ? 1.0
                                                    : prm.order * pow(delta, prm.order - 1.0));
     return 2;
+}
+
+// A pose's map from quadrature points to grid index coordinates in FP32:
+// f = M x + t with M = R_B^T R_A / h, t = (R_B^T (r_A - r_B) - bmin) / h - 1/2.
+// M, t and three fused steps are each rounded to 2^-24 of at most
+// |M|max |x|_1 + |t|max, so f is within e0 + e1 |x|_1 of the FP64 value.
+struct TouchFrame
+{
+    float M[9], t[3], e0, e1;
+};
+
+// Entry `q` of M (0..8) or t (9..11), for threads 0..11.
+__device__ __forceinline__ void set_touch_entry(const GridView& g, const sdfo_body_state& sA,
+                                                const sdfo_body_state& sB, const v3& tl, int q, TouchFrame& f)
+{
+    if (q < 9)
+    {
+        const int a = q / 3, b = q % 3;
+        f.M[q] = (float)((sB.R[a] * sA.R[b] + sB.R[3 + a] * sA.R[3 + b] + sB.R[6 + a] * sA.R[6 + b]) * g.ivoxel[a]);
+    }
+    else if (q < 12)
+    {
+        const int a = q - 9;
+        f.t[a] = (float)(((a == 0 ? tl.x : a == 1 ? tl.y : tl.z) - g.bmin[a]) * g.ivoxel[a] - 0.5);
+    }
+}
+
+__device__ __forceinline__ void set_touch_margin(TouchFrame& f)
+{
+    float m = 0.f;
+#pragma unroll
+    for (int q = 0; q < 9; ++q) m = fmaxf(m, fabsf(f.M[q]));
+    f.e1 = m * 0x1p-21f;
+    f.e0 = fmaxf(fabsf(f.t[0]), fmaxf(fabsf(f.t[1]), fabsf(f.t[2]))) * 0x1p-21f + 0x1p-28f;
+}
+
+enum : int
+{
+    kOutside = 0, // certainly outside the grid
+    kClear = 1,   // certainly inside, in a cell that the surface does not reach
+    kMayTouch = 2 // anything else: the FP64 path decides
+};
+
+__device__ __forceinline__ int touch_status(const GridView& g, const uint32_t* __restrict__ bits, const TouchFrame& f,
+                                            float x, float y, float z)
+{
+    const float e = __fmaf_rn(fabsf(x) + fabsf(y) + fabsf(z), f.e1, f.e0);
+    const int n[3] = {g.nx, g.ny, g.nz};
+    int c[3];
+    bool out = false;
+    float edge = 1.f; // distance to the nearest cell boundary
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+    {
+        const float v = __fmaf_rn(f.M[3 * a], x, __fmaf_rn(f.M[3 * a + 1], y, __fmaf_rn(f.M[3 * a + 2], z, f.t[a])));
+        out = out || v < -e || v > (float)(n[a] - 1) + e;
+        // floor by rounding v - 1/2 at 1.5 2^23 (|v| < 2^20; a point that this
+        // rounds the other way lies on a boundary)
+        const float r = (v - 0.5f) + 12582912.f;
+        c[a] = __float_as_int(r) - 0x4b400000;
+        const float u = v - (r - 12582912.f);
+        edge = fminf(edge, fminf(u, 1.f - u));
+    }
+    const bool cell = !out && edge > e && e < 0.25f && (unsigned)c[0] < (unsigned)(n[0] - 1) &&
+                      (unsigned)c[1] < (unsigned)(n[1] - 1) && (unsigned)c[2] < (unsigned)(n[2] - 1);
+    const int i = cell ? c[0] + n[0] * (c[1] + n[1] * c[2]) : 0;
+    const uint32_t w = __ldg(bits + (i >> 5)); // no branch about it: loads of several points overlap
+    return out ? kOutside : cell && !((w >> (i & 31)) & 1u) ? kClear : kMayTouch;
 }
 
 // Column j of the point's d(f, x f)/d(dx, dtheta), weighted by w.
@@ -246,18 +339,17 @@ __device__ __forceinline__ void jacobian_column(const PointState& st, const sdfo
     col[5] = st.wq * dtq.z;
 }
 
-// One CTA per pose.  Per chunk of 256 quadrature points: every thread
-// evaluates its point (no Hessian) and accumulates F, tau; with JAC the
-// chunk's active points (typically a small fraction) are then compacted in
-// point order into the first threads, which re-evaluate them with the
-// interpolant's Hessian and form the six Jacobian columns -- so only
-// ceil(active / 32) warps run the FP64 derivative code, with full lanes.
+// One CTA per pose.  Without touch bits every thread evaluates its points (no
+// Hessian) and accumulates F, tau, and with JAC the points in contact (typically
+// a small fraction) are listed and evaluated again with the interpolant's
+// Hessian for the six Jacobian columns; with touch bits all of that runs on
+// the listed points alone.
 // Resident CTAs per SM asked of the register allocator (256 threads each).
 #ifndef SDFO_CONTACT_MIN_BLOCKS
 #define SDFO_CONTACT_MIN_BLOCKS 3
 #endif
 #ifndef SDFO_CONTACT_JAC_MIN_BLOCKS
-#define SDFO_CONTACT_JAC_MIN_BLOCKS 2
+#define SDFO_CONTACT_JAC_MIN_BLOCKS 3
 #endif
 
 // Lexicographic (gap, key) minimum for measure_pair's argmin: the reference
@@ -298,20 +390,26 @@ __device__ __forceinline__ int warp_isum(int v)
 
 // EXT: the culled / measuring variant (ContactCull, measures); without it
 // every point is evaluated and no measure is produced.
-template <int MODE, bool SPARSE, int BD, bool JAC, bool EXT>
-__global__ void __launch_bounds__(kContactThreads,
-                                  JAC ? SDFO_CONTACT_JAC_MIN_BLOCKS : SDFO_CONTACT_MIN_BLOCKS)
+// TOUCH: `bits` are the mode's touch bits of a dense grid.  The first pass lists
+// the points that may touch (with JAC alone: the points in contact), the second
+// evaluates the list.
+template <int MODE, bool SPARSE, int BD, bool JAC, bool EXT, bool TOUCH, int T>
+__global__ void __launch_bounds__(T, T == kFewThreads ? 1 : JAC ? SDFO_CONTACT_JAC_MIN_BLOCKS : SDFO_CONTACT_MIN_BLOCKS)
     k_contact(GridView g, const float* __restrict__ qx, const float* __restrict__ qw, int nq,
               const sdfo_body_state* __restrict__ poses, const sdfo_body_state* __restrict__ body_b,
               sdfo_contact_params prm, double* __restrict__ ft, double* __restrict__ jac, ContactCull cull,
-              sdfo_contact_measure* __restrict__ meas)
+              sdfo_contact_measure* __restrict__ meas, const uint32_t* __restrict__ bits)
 {
-    constexpr int kWarps = kContactThreads / 32;
+    constexpr int kWarps = T / 32, kJacPerWarp = kJacSpan / kWarps;
     const int pose = blockIdx.x;
     __shared__ sdfo_body_state sA, sB;
     __shared__ double red[kWarps][6];
     __shared__ double sjac[JAC ? kWarps : 1][JAC ? 36 : 1];
-    __shared__ int s_list[JAC ? kJacSpan : 1];
+    constexpr bool LIST = JAC || TOUCH;
+    __shared__ int s_list[LIST ? kJacSpan : 1];
+    __shared__ int s_act[TOUCH && JAC ? kJacSpan : 1];
+    __shared__ int s_acnt[kWarps];
+    __shared__ TouchFrame s_touch;
     __shared__ int s_wcnt[kWarps];
     __shared__ unsigned s_mask[EXT ? kMaxCullLeaves / 32 : 1];
     __shared__ double s_box[6];
@@ -320,10 +418,14 @@ __global__ void __launch_bounds__(kContactThreads,
     __shared__ int s_cnt[EXT ? kWarps : 1][2];
     __shared__ int s_prefix;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (threadIdx.x == 0)
     {
-        sA = poses[pose];
-        sB = *body_b;
+        // 18 doubles each, one per thread
+        static_assert(sizeof(sdfo_body_state) == 18 * sizeof(double), "a body state is 18 doubles");
+        const int q = (int)threadIdx.x;
+        if (q < 18)
+            reinterpret_cast<double*>(&sA)[q] = __ldg(reinterpret_cast<const double*>(poses + pose) + q);
+        else if (q < 36)
+            reinterpret_cast<double*>(&sB)[q - 18] = __ldg(reinterpret_cast<const double*>(body_b) + q - 18);
     }
     if (JAC)
         for (int t = lane; t < 36; t += 32) sjac[warp][t] = 0.0;
@@ -336,6 +438,14 @@ __global__ void __launch_bounds__(kContactThreads,
     f.vB = V(sB.v[0], sB.v[1], sB.v[2]);
     f.wB = V(sB.w[0], sB.w[1], sB.w[2]);
     f.tl = mulT(sB.R, f.rA - f.rB); // R_B^T (r_A - r_B)
+    TouchFrame tf;
+    if (TOUCH)
+    {
+        set_touch_entry(g, sA, sB, f.tl, (int)threadIdx.x, s_touch);
+        __syncthreads();
+        tf = s_touch;
+        set_touch_margin(tf);
+    }
 
     // broad phase: AABB_BVH.query(bmin_local, bmax_local) (bvh.py:62-80)
     bool full = true;
@@ -356,13 +466,13 @@ __global__ void __launch_bounds__(kContactThreads,
                 enc = enc && s_box[a] <= cull.root[a] && s_box[3 + a] >= cull.root[3 + a];
             s_full = enc ? 1 : 0;
         }
-        for (int w = threadIdx.x; w < (cull.nleaves + 31) / 32; w += kContactThreads) s_mask[w] = 0u;
+        for (int w = threadIdx.x; w < (cull.nleaves + 31) / 32; w += T) s_mask[w] = 0u;
         __syncthreads();
         full = s_full != 0;
         if (!full)
         {
             bool any = false;
-            for (int l = threadIdx.x; l < cull.nleaves; l += kContactThreads)
+            for (int l = threadIdx.x; l < cull.nleaves; l += T)
             {
                 const double* b = cull.leaf_box + 6 * (int64_t)l;
                 const bool skip = b[3] < s_box[0] || b[4] < s_box[1] || b[5] < s_box[2] || b[0] > s_box[3] ||
@@ -383,99 +493,166 @@ __global__ void __launch_bounds__(kContactThreads,
     MinRec best{INFINITY, INT_MAX, -1};
     int nvalid = 0, nactive = 0;
 
-    // Spans of kJacSpan points (one span over all points without the
-    // Jacobian).  First every point's forward; with the Jacobian, each warp
-    // lists its points in contact, in point order, with no barrier.  Then
-    // the span's list is shared out: group k of 32 consecutive entries to
-    // warp k mod 8, so all warps carry the FP64 Jacobian work, and the sums
-    // run in a fixed order (repeated runs are bit-identical).  Block-uniform
-    // trip counts: the barriers and warp reductions below see every thread.
-    for (int s0 = 0; s0 < nq; s0 += JAC ? kJacSpan : nq)
+    // whether the broad phase keeps point i
+    auto kept = [&](int i) {
+        if (!EXT || full) return true;
+        const int l = __ldg(cull.pleaf + i);
+        return ((s_mask[l >> 5] >> (l & 31)) & 1u) != 0;
+    };
+    auto measure_point = [&](int i, double gap) {
+        ++nvalid;
+        if (gap < 0.0) ++nactive;
+        const MinRec r{gap, full ? (cull.porig ? __ldg(cull.porig + i) : i) : i, i};
+        if (less_rec(r, best)) best = r;
+    };
+    auto add_force = [&](const PointState& st) {
+        const v3 tq = cross(st.off, st.fq);
+        acc[0] = fma(st.wq, st.fq.x, acc[0]);
+        acc[1] = fma(st.wq, st.fq.y, acc[1]);
+        acc[2] = fma(st.wq, st.fq.z, acc[2]);
+        acc[3] = fma(st.wq, tq.x, acc[3]);
+        acc[4] = fma(st.wq, tq.y, acc[4]);
+        acc[5] = fma(st.wq, tq.z, acc[5]);
+    };
+
+    // Spans of kJacSpan points (one span over all points when nothing is
+    // listed).  First every point: by its touch bit, or by the forward law; each
+    // warp lists its points, in point order, with no barrier.  Then the span's
+    // list is shared out: group k of 32 consecutive entries to warp k mod 8, so
+    // all warps carry the FP64 work, and the sums run in a fixed order (repeated
+    // runs are bit-identical).  Block-uniform trip counts: the barriers and warp
+    // reductions below see every thread.
+    for (int s0 = 0; s0 < nq; s0 += LIST ? kJacSpan : nq)
     {
-    const int s1 = JAC ? min(nq, s0 + kJacSpan) : nq;
+    const int s1 = LIST ? min(nq, s0 + kJacSpan) : nq;
     int wcnt = 0; // this warp's listed points in the span (warp-uniform)
-    for (int i0 = s0; i0 < s1; i0 += kContactThreads)
+    auto list_point = [&](bool listed, int i) {
+        const unsigned m = __ballot_sync(0xffffffffu, listed);
+        if (listed) s_list[warp * kJacPerWarp + wcnt + __popc(m & ((1u << lane) - 1u))] = i;
+        wcnt += __popc(m);
+    };
+    if constexpr (TOUCH)
     {
-        const int i = i0 + threadIdx.x;
-        bool act = false;
-        if (i < s1)
+        // kAhead points per thread at a time: their loads, and then those of
+        // their bits, are in flight together
+        for (int i0 = s0 + (int)threadIdx.x; i0 - (int)threadIdx.x < s1; i0 += kAhead * T)
         {
-            bool sel = true;
-            if (EXT && !full)
+            float x[kAhead][3];
+            bool in[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
             {
-                const int l = __ldg(cull.pleaf + i);
-                sel = (s_mask[l >> 5] >> (l & 31)) & 1u;
+                const int i = i0 + u * T;
+                in[u] = i < s1 && kept(i);
+#pragma unroll
+                for (int a = 0; a < 3; ++a) x[u][a] = in[u] ? __ldg(qx + 3 * i + a) : 0.f;
             }
-            if (sel)
+            int status[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) status[u] = touch_status(g, bits, tf, x[u][0], x[u][1], x[u][2]);
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+            {
+                if (want_meas && in[u] && status[u] == kClear) ++nvalid;
+                list_point(in[u] && status[u] == kMayTouch, i0 + u * T);
+            }
+        }
+    }
+    else
+    {
+        for (int i0 = s0; i0 < s1; i0 += T)
+        {
+            const int i = i0 + threadIdx.x;
+            bool act = false;
+            if (i < s1 && kept(i))
             {
                 PointState st;
                 double gap = 0.0;
                 const int status =
                     point_state<MODE, SPARSE, BD, false>(g, qx, qw, i, sA, sB, f, prm, narrow, want_meas, st, gap);
-                if (want_meas && status > 0)
-                {
-                    ++nvalid;
-                    if (gap < 0.0) ++nactive;
-                    const MinRec r{gap, full ? (cull.porig ? __ldg(cull.porig + i) : i) : i, i};
-                    if (less_rec(r, best)) best = r;
-                }
+                if (want_meas && status > 0) measure_point(i, gap);
                 act = status == 2 && want_force;
-                if (act)
-                {
-                    const v3 tq = cross(st.off, st.fq);
-                    acc[0] += st.wq * st.fq.x;
-                    acc[1] += st.wq * st.fq.y;
-                    acc[2] += st.wq * st.fq.z;
-                    acc[3] += st.wq * tq.x;
-                    acc[4] += st.wq * tq.y;
-                    acc[5] += st.wq * tq.z;
-                }
+                if (act) add_force(st);
             }
-        }
-        if (JAC)
-        {
-            const unsigned m = __ballot_sync(0xffffffffu, act);
-            if (act) s_list[warp * kJacPerWarp + wcnt + __popc(m & ((1u << lane) - 1u))] = i;
-            wcnt += __popc(m);
+            if (LIST) list_point(act, i);
         }
     }
-    if (JAC)
+    if (LIST)
     {
         if (lane == 0) s_wcnt[warp] = wcnt;
         __syncthreads();
-        int total = 0;
+        // entry e of the warps' lists one after the other
+        auto entry = [&](const int* list, const int* cnt, int e) {
+            int rem = e, src = 0;
 #pragma unroll
-        for (int w = 0; w < kWarps; ++w) total += s_wcnt[w];
-        for (int k = warp; 32 * k < total; k += kWarps) // warp-uniform
-        {
-            const int e = 32 * k + lane;
-            bool mine = e < total;
-            int idx = 0;
-            if (mine)
+            for (int w = 0; w < kWarps; ++w)
             {
-                // entry e of the span's list: warp src's list, position rem
-                int rem = e, src = 0;
-#pragma unroll
-                for (int w = 0; w < kWarps; ++w)
+                const int c = cnt[w];
+                if (src == w && rem >= c)
                 {
-                    const int c = s_wcnt[w];
-                    if (src == w && rem >= c)
-                    {
-                        rem -= c;
-                        ++src;
-                    }
+                    rem -= c;
+                    ++src;
                 }
-                idx = s_list[src * kJacPerWarp + rem];
             }
-            PointState st;
-            double gap = 0.0;
-            mine = mine && point_state<MODE, SPARSE, BD, true>(g, qx, qw, idx, sA, sB, f, prm, narrow, false,
-                                                               st, gap) == 2;
-#pragma unroll 1
-            for (int j = 0; j < 6; ++j)
+            return list[src * kJacPerWarp + rem];
+        };
+        auto entries = [&](const int* cnt) {
+            int total = 0;
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) total += cnt[w];
+            return total;
+        };
+        if constexpr (TOUCH)
+        {
+            const int total = entries(s_wcnt);
+            int acnt = 0;
+            for (int k = warp; 32 * k < total; k += kWarps) // warp-uniform
             {
+                const int e = 32 * k + lane;
+                bool act = false;
+                int idx = 0;
+                if (e < total)
+                {
+                    idx = entry(s_list, s_wcnt, e);
+                    PointState st;
+                    double gap = 0.0;
+                    const int status =
+                        point_state<MODE, SPARSE, BD, false>(g, qx, qw, idx, sA, sB, f, prm, narrow, want_meas, st, gap);
+                    if (want_meas && status > 0) measure_point(idx, gap);
+                    act = status == 2 && want_force;
+                    if (act) add_force(st);
+                }
+                if (JAC)
+                {
+                    const unsigned m = __ballot_sync(0xffffffffu, act);
+                    if (act) s_act[warp * kJacPerWarp + acnt + __popc(m & ((1u << lane) - 1u))] = idx;
+                    acnt += __popc(m);
+                }
+            }
+            if (JAC)
+            {
+                if (lane == 0) s_acnt[warp] = acnt;
+                __syncthreads();
+            }
+        }
+        if constexpr (JAC)
+        {
+            // one column of the Jacobian of 32 points in contact at a time
+            const int* list = TOUCH ? s_act : s_list;
+            const int* cnt = TOUCH ? s_acnt : s_wcnt;
+            const int total = entries(cnt);
+            for (int k = warp; 32 * (k / 6) < total; k += kWarps) // warp-uniform
+            {
+                const int e = 32 * (k / 6) + lane, j = k % 6;
                 double col[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-                if (mine) jacobian_column(st, sB, f, prm, j, col);
+                if (e < total)
+                {
+                    PointState st;
+                    double gap = 0.0;
+                    if (point_state<MODE, SPARSE, BD, true>(g, qx, qw, entry(list, cnt, e), sA, sB, f, prm, narrow,
+                                                            false, st, gap) == 2)
+                        jacobian_column(st, sB, f, prm, j, col);
+                }
 #pragma unroll
                 for (int r = 0; r < 6; ++r)
                 {
@@ -486,6 +663,21 @@ __global__ void __launch_bounds__(kContactThreads,
         }
         __syncthreads(); // s_list and s_wcnt are rewritten by the next span
     }
+    }
+    if (TOUCH && want_meas && __syncthreads_or(best.gap <= 0.0) == 0)
+    {
+        // Clear of the surface: the least gap is not among the listed points
+        // (elsewhere gaps are positive), so every point is measured.
+        best = MinRec{INFINITY, INT_MAX, -1};
+        nvalid = nactive = 0;
+        for (int i = threadIdx.x; i < nq; i += T)
+            if (kept(i))
+            {
+                PointState st;
+                double gap = 0.0;
+                if (point_state<MODE, SPARSE, BD, false>(g, qx, qw, i, sA, sB, f, prm, narrow, true, st, gap) > 0)
+                    measure_point(i, gap);
+            }
     }
     if (want_force)
     {
@@ -539,7 +731,7 @@ __global__ void __launch_bounds__(kContactThreads,
     {
         const int lb = __ldg(cull.pleaf + b.i);
         int part = 0;
-        for (int l = threadIdx.x; l < lb; l += kContactThreads)
+        for (int l = threadIdx.x; l < lb; l += T)
             if ((s_mask[l >> 5] >> (l & 31)) & 1u) part += __ldg(cull.leaf_start + l + 1) - __ldg(cull.leaf_start + l);
         part = warp_isum(part);
         if (lane == 0 && part) atomicAdd(&s_prefix, part);
@@ -599,35 +791,57 @@ struct ContactLaunch
     sdfo_contact_measure* meas;
 };
 
-template <int MODE, bool SPARSE, int BD, bool EXT>
-void launch4(const GridView& v, const ContactLaunch& c, cudaStream_t s)
+template <int MODE, bool SPARSE, int BD, bool EXT, bool TOUCH, int T>
+void launch5(const GridView& v, const ContactLaunch& c, const uint32_t* bits, cudaStream_t s)
 {
     if (c.jac)
-        k_contact<MODE, SPARSE, BD, true, EXT><<<c.np, kContactThreads, 0, s>>>(v, c.qx, c.qw, c.nq, c.pa, c.pb,
-                                                                                c.prm, c.ft, c.jac, c.cull, c.meas);
+        k_contact<MODE, SPARSE, BD, true, EXT, TOUCH, T><<<c.np, T, 0, s>>>(
+            v, c.qx, c.qw, c.nq, c.pa, c.pb, c.prm, c.ft, c.jac, c.cull, c.meas, bits);
     else
-        k_contact<MODE, SPARSE, BD, false, EXT><<<c.np, kContactThreads, 0, s>>>(v, c.qx, c.qw, c.nq, c.pa, c.pb,
-                                                                                 c.prm, c.ft, c.jac, c.cull, c.meas);
+        k_contact<MODE, SPARSE, BD, false, EXT, TOUCH, T><<<c.np, T, 0, s>>>(
+            v, c.qx, c.qw, c.nq, c.pa, c.pb, c.prm, c.ft, c.jac, c.cull, c.meas, bits);
 }
 
-template <int MODE, bool SPARSE, int BD>
-void launch3(const GridView& v, const ContactLaunch& c, cudaStream_t s)
+template <int MODE, bool SPARSE, int BD, bool EXT, bool TOUCH>
+void launch4(const GridView& v, const ContactLaunch& c, const uint32_t* bits, cudaStream_t s)
+{
+    if constexpr (TOUCH)
+    {
+        if (c.np <= current_sm_count())
+        {
+            launch5<MODE, SPARSE, BD, EXT, TOUCH, kFewThreads>(v, c, bits, s);
+            return;
+        }
+    }
+    launch5<MODE, SPARSE, BD, EXT, TOUCH, kContactThreads>(v, c, bits, s);
+}
+
+template <int MODE, bool SPARSE, int BD, bool TOUCH>
+void launch3(const GridView& v, const ContactLaunch& c, const uint32_t* bits, cudaStream_t s)
 {
     if (c.cull.enabled || c.meas)
-        launch4<MODE, SPARSE, BD, true>(v, c, s);
+        launch4<MODE, SPARSE, BD, true, TOUCH>(v, c, bits, s);
     else
-        launch4<MODE, SPARSE, BD, false>(v, c, s);
+        launch4<MODE, SPARSE, BD, false, TOUCH>(v, c, bits, s);
 }
 
 template <int MODE>
 void launch2(const GridView& v, const ContactLaunch& c, cudaStream_t s)
 {
     if (v.layout == SDFO_LAYOUT_DENSE)
-        launch3<MODE, false, 0>(v, c, s);
+    {
+        // The touch bits say where the gap can be <= 0; they leave out points
+        // whose force is k 0^n, so the law needs n > 0.  Views have no bits.
+        const int64_t voxels = (int64_t)v.nx * v.ny * v.nz;
+        if (v.touch && c.prm.order > 0.0 && voxels < (int64_t(1) << 31))
+            launch3<MODE, false, 0, true>(v, c, v.touch + (MODE == SDFO_TRICUBIC ? touch_words(voxels) : 0), s);
+        else
+            launch3<MODE, false, 0, false>(v, c, nullptr, s);
+    }
     else if (v.bd == 8)
-        launch3<MODE, true, 8>(v, c, s);
+        launch3<MODE, true, 8, false>(v, c, nullptr, s);
     else
-        launch3<MODE, true, 0>(v, c, s);
+        launch3<MODE, true, 0, false>(v, c, nullptr, s);
 }
 
 } // namespace

@@ -238,6 +238,7 @@ GridView make_view(const sdfo_grid* g)
     }
     v.xpair = g->d.xpair;
     v.cell8 = g->d.cell8;
+    v.touch = g->d.touch;
     v.ca_stride = g->ca_stride;
     v.ca_count = g->d.ca_count;
     v.ca_phi64 = g->d.ca_phi64;
@@ -329,23 +330,54 @@ namespace {
 // Dense stencil records from the voxel payload: xpair[v] = {phin[v],
 // phin[v+1]} (x neighbour clamped at the last column), cell8[v] = phi of the
 // 8 cell corners (neighbours clamped at the upper faces; cells there are never
-// interpolated because their upper corners are outside the grid).
-__global__ void k_stencil_layouts(const float4* __restrict__ phin, int nx, int ny, int nz,
-                                  float4* __restrict__ xpair, float4* __restrict__ cell8)
+// interpolated because their upper corners are outside the grid), and the
+// touch bits (GridView::touch; cells at the upper faces: 0).
+__global__ void k_stencil_layouts(const float4* __restrict__ phin, int nx, int ny, int nz, float3 h,
+                                  float4* __restrict__ xpair, float4* __restrict__ cell8,
+                                  uint32_t* __restrict__ touch)
 {
-    const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t N = (int64_t)nx * ny * nz;
-    if (v >= N) return;
+    const int64_t at = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t total = (int64_t)nx * ny * nz;
+    const bool live = at < total; // whole warps write the touch words
+    const int64_t v = live ? at : 0;
     const int i = (int)(v % nx), j = (int)((v / nx) % ny), k = (int)(v / ((int64_t)nx * ny));
     const int64_t dx = i + 1 < nx ? 1 : 0;
     const int64_t dy = j + 1 < ny ? nx : 0;
     const int64_t dz = k + 1 < nz ? (int64_t)nx * ny : 0;
-    const float4 a = phin[v];
-    xpair[2 * v] = a;
-    xpair[2 * v + 1] = phin[v + dx];
-    cell8[2 * v] = make_float4(a.x, phin[v + dx].x, phin[v + dy].x, phin[v + dx + dy].x);
-    cell8[2 * v + 1] = make_float4(phin[v + dz].x, phin[v + dx + dz].x, phin[v + dy + dz].x,
-                                   phin[v + dx + dy + dz].x);
+    float4 c[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) c[q] = phin[v + ((q & 1) ? dx : 0) + ((q & 2) ? dy : 0) + ((q & 4) ? dz : 0)];
+    if (live)
+    {
+        xpair[2 * v] = c[0];
+        xpair[2 * v + 1] = c[1];
+        cell8[2 * v] = make_float4(c[0].x, c[1].x, c[2].x, c[3].x);
+        cell8[2 * v + 1] = make_float4(c[4].x, c[5].x, c[6].x, c[7].x);
+    }
+    // Lower bounds of the interpolants.  Trilinear: the least corner.
+    // Tricubic: phi enters with convex weights, and the slope terms of an axis
+    // sum to at most t (1 - t) <= 1/4 of the largest |h n| there.  The margins
+    // cover the FP32 evaluation.
+    float lo = c[0].x, top = 0.f, sx = 0.f, sy = 0.f, sz = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+    {
+        lo = fminf(lo, c[q].x);
+        top = fmaxf(top, fabsf(c[q].x));
+        sx = fmaxf(sx, fabsf(c[q].y));
+        sy = fmaxf(sy, fabsf(c[q].z));
+        sz = fmaxf(sz, fabsf(c[q].w));
+    }
+    const float slope = sx * h.x + sy * h.y + sz * h.z;
+    const bool cell = live && dx != 0 && dy != 0 && dz != 0;
+    const bool lin = cell && !(lo - 0x1p-20f * top > 0.f);
+    const bool cub = cell && !(lo - (0.25f + 0x1p-12f) * slope - 0x1p-16f * (top + slope) > 0.f);
+    const unsigned wl = __ballot_sync(0xffffffffu, lin), wc = __ballot_sync(0xffffffffu, cub);
+    if ((threadIdx.x & 31) == 0 && live)
+    {
+        touch[v >> 5] = wl;
+        touch[touch_words(total) + (v >> 5)] = wc;
+    }
 }
 
 // Sparse stencil records, per stored voxel: neighbours are found through the
@@ -406,8 +438,11 @@ void build_stencil_layouts(sdfo_grid* g, cudaStream_t s)
     {
         if (!g->d.xpair) g->d.xpair = dalloc<float4>((size_t)N * 2);
         if (!g->d.cell8) g->d.cell8 = dalloc<float4>((size_t)N * 2);
+        if (!g->d.touch) g->d.touch = dalloc<uint32_t>((size_t)touch_words(N) * 2);
         k_stencil_layouts<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(
-            g->d.phin, g->info.shape[0], g->info.shape[1], g->info.shape[2], g->d.xpair, g->d.cell8);
+            g->d.phin, g->info.shape[0], g->info.shape[1], g->info.shape[2],
+            make_float3((float)g->info.voxel[0], (float)g->info.voxel[1], (float)g->info.voxel[2]), g->d.xpair,
+            g->d.cell8, g->d.touch);
     }
     else
     {
@@ -449,6 +484,7 @@ sdfo_grid::~sdfo_grid()
     // batched build allocate theirs outside the shared arena)
     device_free(d.xpair);
     device_free(d.cell8);
+    device_free(d.touch);
     if (borrowed) return;
     device_free(d.phin);
     device_free(d.hess6);
@@ -881,6 +917,7 @@ int sdfo_grid_create_view(const sdfo_grid* g, void* d_phin, sdfo_grid** out)
         v->d = g->d;
         v->d.phin = static_cast<float4*>(d_phin);
         v->d.phi64 = v->d.n64 = v->d.w64 = v->d.h64 = nullptr; // export reads the live payload
+        v->d.touch = nullptr;
         v->d.xpair = v->d.cell8 = nullptr; // stencil copies would go stale: read the payload
         v->borrowed = true;
         v->arena = g->arena;

@@ -134,6 +134,7 @@ struct GridStorage
     float2* brick_affine = nullptr;
     float4* xpair = nullptr; // 2 float4 per voxel
     float4* cell8 = nullptr; // 2 float4 per voxel
+    uint32_t* touch = nullptr; // 2 bits per voxel (GridView::touch)
     // contact-aware candidates, `stride` slots per stored voxel: count (u8),
     // phi and normal (FP64 for dense grids, FP32 for sparse ones, as the
     // reference stores them), branch id
@@ -245,6 +246,10 @@ struct GridView
     //   cell8[v] = phi of the 8 corners of cell v       Trilinear: 1 load / query
     const float4* xpair;
     const float4* cell8;
+    // Dense grids, one bit per cell (lower corner v: word v / 32, bit v % 32), or
+    // NULL: whether the interpolated phi can be <= 0 anywhere in the cell,
+    // Trilinear in the first touch_words(voxels) words, Tricubic in the next.
+    const uint32_t* touch;
     // contact-aware candidates (ca_stride == 0: none)
     int ca_stride;
     const uint8_t* ca_count;
@@ -255,6 +260,8 @@ struct GridView
     const int32_t* ca_branch;
 };
 
+inline __host__ __device__ int64_t touch_words(int64_t voxels) { return (voxels + 31) / 32; }
+
 GridView make_view(const sdfo_grid* g);
 // Which sparse 8^3-brick FP32 grids created from now on get x-pair records
 // (2x the payload's memory): 0 those with pools up to 48 MB, 1 all, 2 none
@@ -264,7 +271,7 @@ void set_sparse_pair_records(int mode);
 // FP32-point queries by the persistent walk kernel (query.cu)
 bool query_walk();
 void set_query_walk(bool on);
-// Fills the stencil layouts from phin (grid.cu): dense xpair and cell8;
+// Fills the stencil layouts from phin (grid.cu): dense xpair, cell8 and touch;
 // sparse 8^3 FP32 bricks: xpair as sparse_pair_records() selects.
 void build_stencil_layouts(sdfo_grid* g, cudaStream_t s);
 
