@@ -34,7 +34,7 @@
 // FP32 cannot tell (TouchFrame), and only the listed points take the FP64
 // transform, the gather and the law, shared out over all warps.  4096 poses of
 // a 7,680-point ring about a block's face, a quarter of them in contact: forces
-// and Jacobian 747 -> 299 us (one B200); bound by the latency of the few FP64
+// and Jacobian 750 -> 281 us (one B200); bound by the latency of the few FP64
 // steps of a pose, no longer by the 31 M gathers.
 #include <climits>
 

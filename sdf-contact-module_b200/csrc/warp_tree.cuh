@@ -34,8 +34,9 @@
 // Measured (one B200, fill alone): 34,816-triangle hollow cylinder into
 // 128 x 128 x 64 voxels 8.4 -> 2.0 ms; 327,680-triangle icosphere, 10.6 M
 // voxels of a sparse 512^3 grid, 37.9 -> 8.1 ms.  Bound now by instruction
-// issue: 2.4 of 4 per cycle, about 17,000 per 64 voxels, of which a quarter
-// FP32 and a tenth FP64.
+// issue: 2.8 of 4 per cycle, about 34,000 per 64 voxels, of which a third FP32
+// and a tenth FP64 (81,920 triangles, 256^3).  A triangle-box test ahead of the
+// frame test changed nothing (7.2 against 7.3 ms).
 #pragma once
 
 #include "build_common.cuh"
