@@ -85,7 +85,6 @@ struct WarpTreeView
     RefTreeView ref;
     const float4* node4; // 4 float4 per node: both child boxes, child codes
     const float4* tri4;  // 5 float4 per slot: the triangle in its own frame (k_tri_frames)
-    float frame_m;       // 2^-20 E: the part of a distance's error that does not grow with it
     float bound_abs;     // warp_bound's absolute part, rounded up
     int* heavy;          // first patches of the pairs handed over
     RayBins rays;
@@ -154,9 +153,10 @@ __global__ void k_pack_node4(RefTreeView b, const int* __restrict__ flags, float
 
 // Each triangle in slot order in its own frame: vertex a, the rows of the
 // rotation to (along ab, in the plane across ab towards c, the normal), the
-// length of ab, and unit directions and lengths of ac and bc in the plane.
+// length of ab, unit directions and lengths of ac and bc in the plane, and the
+// part of TriPoint's error that does not depend on the point.
 // Near-degenerate triangles get a negative length of ab: never culled.
-__global__ void k_tri_frames(RefTreeView b, float4* __restrict__ out)
+__global__ void k_tri_frames(RefTreeView b, float frame_m, float4* __restrict__ out)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= b.n) return;
@@ -182,7 +182,8 @@ __global__ void k_tri_frames(RefTreeView b, float4* __restrict__ out)
     o[1] = make_float4((float)x.y, (float)x.z, (float)y.x, (float)y.y);
     o[2] = make_float4((float)y.z, (float)z.x, (float)z.y, (float)z.z);
     o[3] = make_float4((float)lab, (float)dot(uac, x), (float)dot(uac, y), (float)lac);
-    o[4] = make_float4((float)dot(ubc, x), (float)dot(ubc, y), (float)lbc, 0.f);
+    o[4] = make_float4((float)dot(ubc, x), (float)dot(ubc, y), (float)lbc,
+                       __fmaf_ru(__double2float_ru(lab), 0x1p-20f, frame_m));
 }
 
 // ---------------------------------------------------------------------------
@@ -545,10 +546,11 @@ __device__ __forceinline__ float gap2(const float p[3], float lx, float ly, floa
 }
 
 // Triangle s in FP32.  In the triangle's frame the squared distance is z^2
-// plus the planar one.  Errors: p, a and their difference are rounded to
-// 2^-22 E per axis; rotation, unit vectors and products add less than
-// 14 roundings of r = |x| + |y| + |z|.  So the distance is known to within
-// m = 2^-20 (E + r).
+// plus the planar one.  Errors, in units of 2^-24: p and a are rounded to E per
+// axis; their difference, the rotation, the segments of ab and ac and the root
+// add less than 17 r, r = |x| + |y| + |z|; the segment of bc, 8 |ab|.  So the
+// distance to the plane, to an edge's line or to a segment is known to within
+// m = 2^-20 (E + r + |ab|).
 struct TriFrame
 {
     float4 q0, q1, q2, q3, q4;
@@ -560,26 +562,29 @@ struct TriFrame
 // triangle's plane and the lines of its edges (need()), then the distance.
 struct TriPoint
 {
-    float x, y, z, m, eac, ebc, out;
-    __device__ __forceinline__ TriPoint(const WarpTreeView& t, const TriFrame& f, const float p[3])
+    float x, y, z, m, eac, ebc, side;
+    __device__ __forceinline__ TriPoint(const TriFrame& f, const float p[3])
     {
         const float dx = p[0] - f.q0.x, dy = p[1] - f.q0.y, dz = p[2] - f.q0.z;
         x = __fmaf_rn(f.q0.w, dx, __fmaf_rn(f.q1.x, dy, f.q1.y * dz));
         y = __fmaf_rn(f.q1.z, dx, __fmaf_rn(f.q1.w, dy, f.q2.x * dz));
         z = __fmaf_rn(f.q2.y, dx, __fmaf_rn(f.q2.z, dy, f.q2.w * dz));
-        m = __fmaf_rn(fabsf(x) + fabsf(y) + fabsf(z), 0x1p-20f, t.frame_m);
+        m = __fmaf_rn(fabsf(x) + fabsf(y) + fabsf(z), 0x1p-20f, f.q4.w);
         // signed distances outward of the edges ab, ac, bc
         eac = __fmaf_rn(f.q3.y, y, -(f.q3.z * x));
         ebc = __fmaf_rn(f.q4.y, x - f.q3.x, -(f.q4.x * y));
-        out = fmaxf(fmaxf(-y, fmaxf(eac, ebc)), 0.f);
+        side = fmaxf(-y, fmaxf(eac, ebc));
     }
     __device__ __forceinline__ bool need(const TriFrame& f, float bound) const
     {
-        const float lz = fmaxf(fabsf(z) - m, 0.f), lo = fmaxf(out - m, 0.f);
+        const float lz = fmaxf(fabsf(z) - m, 0.f), lo = fmaxf(side - m, 0.f);
         return f.whole() || !(__fmaf_rn(lz, lz, lo * lo) > bound);
     }
     // Bounds of the squared distance; false: the triangle cannot matter.
-    // Otherwise `bound` is lowered to what this triangle attains.
+    // Otherwise `bound` is lowered to what this triangle attains: the distance
+    // to its plane only where the point is inside its edges by more than their
+    // error, else that to the nearest segment.  (At a needle's tip the edges'
+    // signs are lost in rounding well outside the triangle.)
     __device__ __forceinline__ bool reaches(const WarpTreeView& t, const TriFrame& f, float& bound, float& low) const
     {
         // planar distance: 0 inside, else to the nearest of the three segments
@@ -589,13 +594,13 @@ struct TriPoint
         const float tbc = __fmaf_rn(f.q4.x, xb, f.q4.y * y), sbc = tbc - fminf(fmaxf(tbc, 0.f), f.q4.z);
         const float d2 = fminf(__fmaf_rn(sab, sab, y * y), fminf(__fmaf_rn(sac, sac, eac * eac),
                                                                 __fmaf_rn(sbc, sbc, ebc * ebc)));
-        const float d = sqrtf(__fmaf_rn(z, z, out > 0.f ? d2 : 0.f));
+        const float d = sqrtf(__fmaf_rn(z, z, side > 0.f ? d2 : 0.f));
         low = fmaxf(d - m, 0.f);
         low = f.whole() ? 0.f : low * low;
         if (low > bound) return false;
         if (!f.whole())
         {
-            const float up = d + m;
+            const float up = (side > 0.f || side < -m ? d : sqrtf(__fmaf_rn(z, z, d2))) + m;
             bound = fminf(bound, __fmaf_ru(__fmul_ru(up, up), 1.f + 0x1p-15f, t.bound_abs));
         }
         return true;
@@ -684,7 +689,7 @@ __device__ __forceinline__ bool warp_search(const WarpTreeView& t, int node, int
             for (int s = meta.z; s < meta.z + meta.w; ++s)
             {
                 const TriFrame f(tris + 5 * (s - meta.z));
-                const TriPoint u(t, f, pf[0]), v(t, f, pf[1]);
+                const TriPoint u(f, pf[0]), v(f, pf[1]);
                 if (!__any_sync(0xffffffffu, u.need(f, bound[0]) || v.need(f, bound[1]))) continue;
 #pragma unroll
                 for (int k = 0; k < 2; ++k)
@@ -1174,7 +1179,7 @@ struct DeviceWarpTree
         SDFO_CHECK_LAUNCH();
         k_pack_node4<<<(tree.nnodes + T - 1) / T, T, 0, s>>>(tree, flags.get(), node4.get());
         SDFO_CHECK_LAUNCH();
-        k_tri_frames<<<(n + T - 1) / T, T, 0, s>>>(tree, tri4.get());
+        k_tri_frames<<<(n + T - 1) / T, T, 0, s>>>(tree, (float)std::ldexp(extent, -20), tri4.get());
         SDFO_CHECK_LAUNCH();
         k_ray_count<<<(n + T - 1) / T, T, 0, s>>>(tree, v.rays, extent, rec.get(), counts.get(), state.get());
         SDFO_CHECK_LAUNCH();
@@ -1187,7 +1192,6 @@ struct DeviceWarpTree
         SDFO_CHECK_LAUNCH();
         v.node4 = node4.get();
         v.tri4 = tri4.get();
-        v.frame_m = (float)std::ldexp(extent, -20);
         v.bound_abs = (float)(tree.cull_abs * (1.0 + 0x1p-15));
         v.rays.rec = rec.get();
         v.rays.off = off.get();
