@@ -27,20 +27,21 @@ class SDFQuery(torch.autograd.Function):
         g = grid if payload is None else grid.view(payload)
         ctx.grid = g
         ctx.mode = mode
-        ctx.saved = None
+        ctx.names = ()
         if points.dtype == torch.float32 and points.is_cuda:
             pts = points.detach().contiguous().reshape(-1, 3)
             if ctx.needs_input_grad[0]:
                 out = g.query_linearize(pts, mode=mode)
-                # aliases without the graph: an output kept on its own node would
-                # be a reference cycle, and every call's tensors would stay until
-                # the garbage collector runs (2M points: a pass 1.2 ms, most of it
-                # fresh device allocations, against 0.25 ms of kernels)
-                ctx.saved = dict(grad=out["grad"].detach(), hess6=out["hess6"], valid=out["valid"])
+                ctx.names = ("grad", "hess6", "valid")
             else:
                 out = g.query_tensors(pts, mode=mode, valid=True)
-                ctx.saved = dict(valid=out["valid"])
-            ctx.save_for_backward(points)
+                ctx.names = ("valid",)
+            # not as attributes: an output kept on its own node would be a
+            # reference cycle, and every call's tensors would stay until the
+            # garbage collector runs (2M points: a pass 1.2 ms, most of it fresh
+            # device allocations, against 0.25 ms of kernels); and a caller that
+            # changes the returned gradient in place has to hear of it
+            ctx.save_for_backward(points, *(out[k] for k in ctx.names))
             return out["gap"], out["grad"]
         out = g.query_tensors(points, mode=mode, valid=False)
         ctx.save_for_backward(points)
@@ -48,7 +49,7 @@ class SDFQuery(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dgap, dgrad):
-        (points,) = ctx.saved_tensors
+        points, *saved = ctx.saved_tensors
         g = ctx.grid
         need_p = ctx.needs_input_grad[0]
         need_v = ctx.needs_input_grad[1]
@@ -56,8 +57,8 @@ class SDFQuery(torch.autograd.Function):
         if need_v:
             dgrid = torch.zeros((g.stored_voxels, 4), dtype=torch.float32, device=points.device)
         pts32 = points.detach().to(torch.float32).contiguous().reshape(-1, 3)
-        if ctx.saved is not None:
-            dpts = g.query_backward_saved(pts32, ctx.saved, dgap, dgrad, mode=ctx.mode,
+        if saved:
+            dpts = g.query_backward_saved(pts32, dict(zip(ctx.names, saved)), dgap, dgrad, mode=ctx.mode,
                                           dgrid=dgrid, want_points=need_p)
         else:
             dpts = g.query_backward(pts32, dgap, dgrad, mode=ctx.mode, dgrid=dgrid,
