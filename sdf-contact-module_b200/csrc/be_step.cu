@@ -46,8 +46,9 @@
 // gather) and FP64 issue, so they leave out what cannot matter: measure_pass
 // samples in FP64 only where FP32 bounds do not rule a point out, and an
 // evaluation from the cache reads 8 bytes of a point that stays clear.  2048
-// rings (7,680 points) about the slab, half touching, two steps: 12.6 -> 9.4 ms
-// (the bounds 4 %, the cached evaluation the rest), identical states.
+// rings (7,680 points) about the slab, half touching, two steps: 12.3 -> 8.0 ms,
+// identical states.  Small point sets take kernels without the bounds
+// (kBoundPoints): with them, even unused, a step of 480 points was 7 % slower.
 //
 // Control flow: every thread runs the same loops and branches; decisions and
 // all scalar state live in shared memory, written by thread 0 between
@@ -109,6 +110,11 @@ constexpr int kJac = 72; // Jp (36) then Jv (36), row-major 6x6 each
 // up to kPrefCap entries (32,768 points at 256 threads), larger point sets
 // take the per-chunk block scan.
 constexpr int kPrefCap = 1024;
+// Points from which a scene's CTA takes the FP32 bounds of measure_pass (a warp
+// per scene: always, 1.00 to 1.34 times as fast).  2048 drops, two steps, 256
+// threads: 480 points 0.895 ms with bounds, 0.875 without; 1,536 points 1.036
+// and 1.086; 7,680 points 2.49 and 3.11.
+constexpr int kBoundPoints = 1536;
 
 struct MinRec
 {
@@ -533,8 +539,8 @@ __device__ void point_jacobian(const BeView& b, const double rg[3], const double
 // (every lane of the warp calls it; inactive lanes pass w = 0).  Column by
 // column: for each of the 12 columns the 6 entries are warp-summed and lane
 // 0 adds them to its row in chunk order.
-__device__ void add_point_jacobian(double* row, double w, const double Gt[9], const double U[9],
-                                   const double off[3], const double fq[3], const double wA[3])
+__device__ __noinline__ void add_point_jacobian(double* row, double w, const double Gt[9], const double U[9],
+                                                const double off[3], const double fq[3], const double wA[3])
 {
     const int lane = (int)(threadIdx.x & 31);
     double Ox[9], Wx[9], Fx[9], A[9], UW[9];
@@ -577,8 +583,8 @@ __device__ void add_point_jacobian(double* row, double w, const double Gt[9], co
 
 // SDFContactEngine.evaluate for s.cur with the cache (F, tau into shared);
 // JAC: also Jp and Jv (row 0 of s.jred) for the exact tangent.
-template <bool W, bool JAC>
-__device__ void eval_pass(const BeView& b, Shared& s)
+template <bool W, bool JAC, bool EXACT>
+__device__ __forceinline__ void eval_body(const BeView& b, Shared& s)
 {
     broad_phase<W>(b, s);
     const double narrow = b.cull ? b.narrow : INFINITY;
@@ -607,7 +613,7 @@ __device__ void eval_pass(const BeView& b, Shared& s)
             if (lane == 0)
             {
                 s.pref[k * nw + warp] = __popc(bal);
-                s.fbal[k * nw + warp] = bal;
+                if (!EXACT) s.fbal[k * nw + warp] = bal;
             }
         }
         Grp<W>::sync();
@@ -669,11 +675,11 @@ __device__ void eval_pass(const BeView& b, Shared& s)
             double X[3], w = 0.0, Y[3];
             bool f = false;
             int pos;
-            if (fast)
+            if (!EXACT && fast)
             {
                 // the flags and positions of the counting loop
                 const unsigned bal = s.fbal[k * nw + warp];
-                if (bal == 0u && !JAC) continue; // warp-uniform
+                if (bal == 0u) continue; // warp-uniform
                 f = (bal >> lane) & 1u;
                 pos = s.pref[k * nw + warp] + __popc(bal & lt);
                 if (f && use && b.cg[base_c + pos] > clear) f = false;
@@ -686,9 +692,14 @@ __device__ void eval_pass(const BeView& b, Shared& s)
                     to_sdf(s, X, Y);
                     f = fabs(Y[2]) < narrow;
                 }
-                int total;
-                pos = base + chunk_scan<W>(s, f, total);
-                base += total;
+                if (fast) // the same flags as the counting loop: position from the prefix
+                    pos = s.pref[k * nw + warp] + __popc(__ballot_sync(0xffffffffu, f) & lt);
+                else
+                {
+                    int total;
+                    pos = base + chunk_scan<W>(s, f, total);
+                    base += total;
+                }
             }
             bool act = false;
             double fq[3] = {0.0, 0.0, 0.0}, off[3] = {0.0, 0.0, 0.0};
@@ -722,7 +733,7 @@ __device__ void eval_pass(const BeView& b, Shared& s)
                         b.cgrad[3 * ci + 1] = gr[1];
                         b.cgrad[3 * ci + 2] = gr[2];
                         b.cvalid[ci] = valid ? 1 : 0;
-                        gm = fmax(gm, fabs(gr[0]) + fabs(gr[1]) + fabs(gr[2]));
+                        if (!W && !EXACT) gm = fmax(gm, fabs(gr[0]) + fabs(gr[1]) + fabs(gr[2]));
                     }
                 }
                 const double delta = -g > 0.0 ? -g : 0.0;
@@ -777,7 +788,7 @@ __device__ void eval_pass(const BeView& b, Shared& s)
                 add_point_jacobian(jrow, act ? w : 0.0, Gt, U, off, fq, s.cur.w);
             }
         }
-        if (store)
+        if (!W && !EXACT && store)
         {
             for (int o = 16; o > 0; o >>= 1) gm = fmax(gm, __shfl_xor_sync(0xffffffffu, gm, o));
             if (lane == 0) s.mins[warp].gap = gm;
@@ -786,7 +797,8 @@ __device__ void eval_pass(const BeView& b, Shared& s)
         if (Grp<W>::rank() == 0 && store)
         {
             double g = 0.0;
-            for (int k = 0; k < nw; ++k) g = fmax(g, s.mins[k].gap);
+            if (!W && !EXACT)
+                for (int k = 0; k < nw; ++k) g = fmax(g, s.mins[k].gap);
             s.gmax = g;
             for (int a = 0; a < 3; ++a) s.c_tref[a] = tsdf[a];
             s.c_len = L;
@@ -817,6 +829,25 @@ __device__ void eval_pass(const BeView& b, Shared& s)
     Grp<W>::sync();
 }
 
+// A call of its own (as measure_pass and add_point_jacobian are): inlined into
+// the step, the passes share its registers and spill in their loops.  2048 rings
+// of 7,680 points about the slab, two steps: 9.2 ms inlined, 8.0 as calls.  The
+// warp-per-scene reference step measured 3 % faster inlined.
+template <bool W, bool JAC, bool EXACT>
+__device__ __noinline__ void eval_call(const BeView& b, Shared& s)
+{
+    eval_body<W, JAC, EXACT>(b, s);
+}
+
+template <bool W, bool JAC, bool EXACT>
+__device__ __forceinline__ void eval_pass(const BeView& b, Shared& s)
+{
+    if constexpr (W && !EXACT)
+        eval_body<W, JAC, EXACT>(b, s);
+    else
+        eval_call<W, JAC, EXACT>(b, s);
+}
+
 // measure_pair for s.cur (contacts_sdf.py:171-214): m_gap, m_pen, m_vn,
 // m_active, m_valid.
 //
@@ -824,43 +855,24 @@ __device__ void eval_pass(const BeView& b, Shared& s)
 // bounds tell for almost every point that it is neither: the FP64 sample runs
 // only where the lower bound does not exceed the least upper bound met, or
 // where the bounds straddle 0.  The search starts from the upper bound of the
-// point that the step's previous measure found nearest (s.mi); the first
-// measure of a step finds one in an FP32 pass.  Every point that attains the
-// least FP64 gap is sampled, so gap, index and counts are those of sampling
-// all.  m_valid: not 0 when some point is inside the grid.
-template <bool W>
-__device__ void measure_pass(const BeView& b, Shared& s)
+// point that the step's previous measure found nearest (s.mi), where there is
+// one.  Every point that attains the least FP64 gap is sampled, so gap, index
+// and counts are those of sampling all.  m_valid: not 0 when some point is
+// inside the grid.
+template <bool W, bool BOUNDS>
+__device__ __noinline__ void measure_pass(const BeView& b, Shared& s)
 {
     broad_phase<W>(b, s);
     MinRec best{INFINITY, INT_MAX, -1};
     int nv = 0, na = 0;
-    const bool bounds = b.g.cell8 != nullptr;
     float least = INFINITY; // no gap below it is needed
     Frame32 fr;
-    if (bounds)
+    if (BOUNDS)
     {
         frame32(b, s, fr);
-        int seed = s.mi;
-        if (seed < 0)
-        {
-            for (int i = Grp<W>::rank(); i < b.nq; i += Grp<W>::size())
-            {
-                double X[3], w;
-                float g, eps;
-                if (point_at(b, s, i, X, w) && gap32(b, fr, X, g, eps) == kInside32) least = fminf(least, g + eps);
-            }
-            for (int o = 16; o > 0; o >>= 1) least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
-            if ((threadIdx.x & 31) == 0) s.mins[Grp<W>::warp()].gap = (double)least;
-            Grp<W>::sync();
-            for (int k = 0; k < Grp<W>::warps(); ++k) least = fminf(least, (float)s.mins[k].gap);
-            Grp<W>::sync();
-        }
-        else
-        {
-            double X[3], w;
-            float g, eps;
-            if (point_at(b, s, seed, X, w) && gap32(b, fr, X, g, eps) == kInside32) least = g + eps;
-        }
+        double X[3], w;
+        float g, eps;
+        if (s.mi >= 0 && point_at(b, s, s.mi, X, w) && gap32(b, fr, X, g, eps) == kInside32) least = g + eps;
     }
     // ties of the minimum go to the first kept point; the list index orders
     // kept points as their positions among the kept points do, so it serves
@@ -870,7 +882,7 @@ __device__ void measure_pass(const BeView& b, Shared& s)
         double X[3], w, Y[3];
         const int i = c0 + Grp<W>::rank();
         if (!point_at(b, s, i, X, w)) continue;
-        if (bounds)
+        if (BOUNDS)
         {
             float g32, eps;
             const int k = gap32(b, fr, X, g32, eps);
@@ -994,7 +1006,7 @@ __device__ void kinematic(const Body& q0, const double V[6], double dt, Body& ou
 
 // _residual at V = z (implicit_be.py:536-604): s.res, s.err, s.Iw, s.cur;
 // JAC: also the contact Jacobians of the exact tangent (s.jred).
-template <bool W, bool JAC>
+template <bool W, bool JAC, bool EXACT>
 __device__ void residual(const BeView& b, Shared& s, const double* z, double dt, bool allowed)
 {
     if (Grp<W>::rank() == 0)
@@ -1003,7 +1015,7 @@ __device__ void residual(const BeView& b, Shared& s, const double* z, double dt,
         s.n_resid += 1;
     }
     Grp<W>::sync();
-    if (allowed) eval_pass<W, JAC>(b, s);
+    if (allowed) eval_pass<W, JAC, EXACT>(b, s);
     if (Grp<W>::rank() == 0)
     {
         double RI[9];
@@ -1172,7 +1184,7 @@ __device__ void step_be(const BeView& b, Shared& s, const Body* src, Body* dst, 
         s.n_solves += 1;
     }
     Grp<W>::sync();
-    residual<W, EXACT>(b, s, s.z, dt, allowed);
+    residual<W, EXACT, EXACT>(b, s, s.z, dt, allowed);
     for (int it = 0; it < b.p.max_iter; ++it)
     {
         if (s.err < b.p.tol) break;
@@ -1235,7 +1247,7 @@ __device__ void step_be(const BeView& b, Shared& s, const Body* src, Body* dst, 
             {
                 if (Grp<W>::rank() < 6) s.zt[Grp<W>::rank()] = s.z[Grp<W>::rank()] + alphas[k] * s.dz[Grp<W>::rank()];
                 Grp<W>::sync();
-                residual<W, false>(b, s, s.zt, dt, allowed);
+                residual<W, false, EXACT>(b, s, s.zt, dt, allowed);
                 if (Grp<W>::rank() == 0)
                 {
                     double nr = 0.0;
@@ -1256,7 +1268,7 @@ __device__ void step_be(const BeView& b, Shared& s, const Body* src, Body* dst, 
             for (int a = 0; a < 6; ++a) s.z[a] = s.z[a] + alpha * s.dz[a];
         }
         Grp<W>::sync();
-        residual<W, EXACT>(b, s, s.z, dt, allowed);
+        residual<W, EXACT, EXACT>(b, s, s.z, dt, allowed);
     }
     if (Grp<W>::rank() == 0)
     {
@@ -1270,12 +1282,12 @@ __device__ void step_be(const BeView& b, Shared& s, const Body* src, Body* dst, 
     Grp<W>::sync();
 }
 
-template <bool W>
+template <bool W, bool BOUNDS>
 __device__ void measure_body(const BeView& b, Shared& s, const Body& body)
 {
     if (Grp<W>::rank() == 0) s.cur = body;
     Grp<W>::sync();
-    measure_pass<W>(b, s);
+    measure_pass<W, BOUNDS>(b, s);
 }
 
 __device__ __forceinline__ bool region_active(int ph)
@@ -1341,7 +1353,7 @@ constexpr int jac_smem_bytes() { return (T / 32) * kJac * (int)sizeof(double); }
 
 // T threads per CTA; W: one warp per scene (T / 32 scenes per CTA), else
 // the whole CTA on one scene.
-template <int T, bool W, bool EXACT>
+template <int T, bool W, bool EXACT, bool BOUNDS>
 __global__ void __launch_bounds__(T, (W || T == 256) ? 3 : 4) k_be_step(BeView b, sdfo_be_scene* __restrict__ scenes, int n,
                                                 const double* __restrict__ dt_req, double* __restrict__ h_out,
                                                 const double* __restrict__ t_end, double dt_max,
@@ -1399,7 +1411,7 @@ __global__ void __launch_bounds__(T, (W || T == 256) ? 3 : 4) k_be_step(BeView b
         return; // nothing to do for this scene (finished)
     }
     // _activate_initially_penetrating_regions
-    measure_body<W>(b, s, s.q);
+    measure_body<W, BOUNDS>(b, s, s.q);
     if (Grp<W>::rank() == 0)
     {
         s.last_gap = s.m_gap;
@@ -1419,7 +1431,7 @@ __global__ void __launch_bounds__(T, (W || T == 256) ? 3 : 4) k_be_step(BeView b
     if (s.phase == kInactive && h_cap > 0.0)
     {
         step_be<W, EXACT>(b, s, &s.q, &s.tr, h_cap, false);
-        measure_body<W>(b, s, s.tr);
+        measure_body<W, BOUNDS>(b, s, s.tr);
         if (Grp<W>::rank() == 0)
             s.flag = (s.m0_gap > 0.0 && (s.m_gap <= 0.0 || s.m_pen > p.pen_max)) ? 1 : 0;
         Grp<W>::sync();
@@ -1441,7 +1453,7 @@ __global__ void __launch_bounds__(T, (W || T == 256) ? 3 : 4) k_be_step(BeView b
                 if (s.hit) break;
                 const double mid = 0.5 * (s.lo + s.hi);
                 step_be<W, EXACT>(b, s, &s.q, &s.tr, mid, false);
-                measure_body<W>(b, s, s.tr);
+                measure_body<W, BOUNDS>(b, s, s.tr);
                 if (Grp<W>::rank() == 0)
                 {
                     if (s.m_gap <= 0.0 || s.m_pen > p.pen_max)
@@ -1463,7 +1475,7 @@ __global__ void __launch_bounds__(T, (W || T == 256) ? 3 : 4) k_be_step(BeView b
                 }
                 Grp<W>::sync();
                 step_be<W, EXACT>(b, s, &s.q, &s.tr, s.hi, false);
-                measure_body<W>(b, s, s.tr);
+                measure_body<W, BOUNDS>(b, s, s.tr);
                 if (Grp<W>::rank() == 0) s.hm_pen = s.m_pen;
                 Grp<W>::sync();
             }
@@ -1493,7 +1505,7 @@ __global__ void __launch_bounds__(T, (W || T == 256) ? 3 : 4) k_be_step(BeView b
             if (s.hit) s.min_dt_hits += 1;
         }
         Grp<W>::sync();
-        measure_body<W>(b, s, s.q);
+        measure_body<W, BOUNDS>(b, s, s.q);
         if (Grp<W>::rank() == 0)
         {
             s.last_gap = s.m_gap;
@@ -1505,7 +1517,7 @@ __global__ void __launch_bounds__(T, (W || T == 256) ? 3 : 4) k_be_step(BeView b
     {
         h = h_cap;
         step_be<W, EXACT>(b, s, &s.q, &s.q, h, region_active(s.phase));
-        measure_body<W>(b, s, s.q);
+        measure_body<W, BOUNDS>(b, s, s.q);
         if (Grp<W>::rank() == 0) refresh(b, s);
     }
     Grp<W>::sync();
@@ -1600,24 +1612,30 @@ namespace {
 void launch_step(const sdfo_be_stepper* st, sdfo_be_scene* scenes, int64_t n, const double* dt, double* h,
                  const double* t_end, double dt_max, int* unfinished, cudaStream_t s)
 {
-#define SDFO_BE_LAUNCH(EX)                                                                                  \
+#define SDFO_BE_LAUNCH(T, W, EX, BD)                                                                        \
+    k_be_step<T, W, EX, BD><<<(unsigned)(W ? (n + 7) / 8 : n), T, EX ? jac_smem_bytes<T>() : 0, s>>>(       \
+        st->view, scenes, (int)n, dt, h, t_end, dt_max, unfinished)
+#define SDFO_BE_LAUNCH_THREADS(EX)                                                                          \
     if (st->threads == 32)                                                                                  \
-        k_be_step<256, true, EX><<<(unsigned)((n + 7) / 8), 256, EX ? jac_smem_bytes<256>() : 0, s>>>(     \
-            st->view, scenes, (int)n, dt, h, t_end, dt_max, unfinished);                                    \
+        SDFO_BE_LAUNCH(256, true, EX, true);                                                                \
+    else if (st->threads == 128 && bounds)                                                                  \
+        SDFO_BE_LAUNCH(128, false, EX, true);                                                               \
     else if (st->threads == 128)                                                                            \
-        k_be_step<128, false, EX><<<(unsigned)n, 128, EX ? jac_smem_bytes<128>() : 0, s>>>(                 \
-            st->view, scenes, (int)n, dt, h, t_end, dt_max, unfinished);                                    \
+        SDFO_BE_LAUNCH(128, false, EX, false);                                                              \
+    else if (bounds)                                                                                        \
+        SDFO_BE_LAUNCH(256, false, EX, true);                                                               \
     else                                                                                                    \
-        k_be_step<256, false, EX><<<(unsigned)n, 256, EX ? jac_smem_bytes<256>() : 0, s>>>(                 \
-            st->view, scenes, (int)n, dt, h, t_end, dt_max, unfinished);
+        SDFO_BE_LAUNCH(256, false, EX, false);
+    const bool bounds = st->view.nq >= kBoundPoints;
     if (st->view.p.tangent == SDFO_BE_TANGENT_EXACT)
     {
-        SDFO_BE_LAUNCH(true)
+        SDFO_BE_LAUNCH_THREADS(true)
     }
     else
     {
-        SDFO_BE_LAUNCH(false)
+        SDFO_BE_LAUNCH_THREADS(false)
     }
+#undef SDFO_BE_LAUNCH_THREADS
 #undef SDFO_BE_LAUNCH
     SDFO_CHECK_LAUNCH();
 }
@@ -1724,7 +1742,7 @@ int sdfo_be_stepper_create(const sdfo_contact_pair* pair, const sdfo_contact_par
         *out = nullptr;
         SDFO_REQUIRE(pair->grid != nullptr, SDFO_ERR_INVALID_ARGUMENT, "pair was created without a grid");
         const sdfo_grid* g = pair->grid;
-        SDFO_REQUIRE(g->info.layout == SDFO_LAYOUT_DENSE && g->d.phi64 != nullptr, SDFO_ERR_UNSUPPORTED,
+        SDFO_REQUIRE(g->info.layout == SDFO_LAYOUT_DENSE && g->d.phi64 && g->d.cell8, SDFO_ERR_UNSUPPORTED,
                      "BE stepping samples a dense grid's FP64 values (build, load or create it from FP64 data)");
         SDFO_REQUIRE(max_scenes > 0 && max_scenes <= 0x7fffffff, SDFO_ERR_INVALID_ARGUMENT, "bad scene count");
         SDFO_REQUIRE(params->max_iter >= 0 && params->max_toi_bisect_iter >= 0, SDFO_ERR_INVALID_ARGUMENT,
@@ -1783,12 +1801,14 @@ int sdfo_be_stepper_create(const sdfo_contact_pair* pair, const sdfo_contact_par
         if (params->tangent == SDFO_BE_TANGENT_EXACT)
         {
             // static + dynamic shared memory above 48 KB needs the opt-in
-            SDFO_CUDA(cudaFuncSetAttribute(k_be_step<256, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           jac_smem_bytes<256>()));
-            SDFO_CUDA(cudaFuncSetAttribute(k_be_step<256, false, true>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, jac_smem_bytes<256>()));
-            SDFO_CUDA(cudaFuncSetAttribute(k_be_step<128, false, true>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, jac_smem_bytes<128>()));
+            auto opt_in = [](const void* kernel, int bytes) {
+                SDFO_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+            };
+            opt_in((const void*)k_be_step<256, true, true, true>, jac_smem_bytes<256>());
+            opt_in((const void*)k_be_step<256, false, true, true>, jac_smem_bytes<256>());
+            opt_in((const void*)k_be_step<256, false, true, false>, jac_smem_bytes<256>());
+            opt_in((const void*)k_be_step<128, false, true, true>, jac_smem_bytes<128>());
+            opt_in((const void*)k_be_step<128, false, true, false>, jac_smem_bytes<128>());
         }
         b.stats = dalloc<unsigned long long>(3);
         SDFO_CUDA(cudaMemset(b.stats, 0, 3 * sizeof(unsigned long long)));
