@@ -57,7 +57,7 @@
 #include <climits>
 #include <cstring>
 
-#include "sdfo_internal.cuh"
+#include "place32.cuh"
 
 namespace sdfo {
 namespace {
@@ -268,67 +268,31 @@ __device__ bool sample64(const BeView& b, const double Y[3], double& g, double g
 }
 
 // The pass's pose as a map from points to grid index coordinates in FP32, for
-// bounds of a point's gap ahead of the FP64 sample.  x, M, t and three fused
-// steps are each rounded to 2^-24 of at most |M|max |x|_1 + |t|max, so a
-// coordinate is within e0 + e1 |x|_1 of the FP64 one.
-struct Frame32
+// bounds of a point's gap ahead of the FP64 sample.
+__device__ __forceinline__ void frame32(const BeView& b, const Shared& s, Place32& f)
 {
-    float M[9], t[3], e0, e1;
-};
-
-__device__ __forceinline__ void frame32(const BeView& b, const Shared& s, Frame32& f)
-{
-    float m = 0.f, q = 0.f;
+    double far = 0.0;
 #pragma unroll
     for (int a = 0; a < 3; ++a)
     {
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-        {
-            f.M[3 * a + c] = (float)(s.Rs[3 * a + c] * b.g.ivoxel[a]);
-            m = fmaxf(m, fabsf(f.M[3 * a + c]));
-        }
+        for (int c = 0; c < 3; ++c) f.M[3 * a + c] = (float)(s.Rs[3 * a + c] * b.g.ivoxel[a]);
         f.t[a] = (float)((s.tl[a] - b.g.bmin[a]) * b.g.ivoxel[a] - 0.5);
-        q = fmaxf(q, fabsf(f.t[a]));
+        far = fmax(far, (fabs(s.tl[a]) + fabs(b.g.bmin[a])) * b.g.ivoxel[a]);
     }
-    f.e0 = q * 0x1p-20f + 0x1p-28f;
-    f.e1 = m * 0x1p-20f;
+    f.set_margin(far);
 }
-
-enum : int
-{
-    kOut32 = 0,    // certainly outside the grid
-    kInside32 = 1, // certainly inside; the FP64 gap lies in g -+ eps
-    kUnsure32 = 2  // only the FP64 sample can tell
-};
 
 // The gap at X from the cell's FP32 corner record.  A coordinate off by e
 // moves the interpolant by at most e times the corners' spread per axis; the
 // corners and the interpolation are rounded to less than 2^-20 of the largest.
-__device__ __forceinline__ int gap32(const BeView& b, const Frame32& f, const double X[3], float& g, float& eps)
+__device__ __forceinline__ int gap32(const BeView& b, const Place32& f, const double X[3], float& g, float& eps)
 {
-    const float x = (float)X[0], y = (float)X[1], z = (float)X[2];
-    const float e = __fmaf_rn(fabsf(x) + fabsf(y) + fabsf(z), f.e1, f.e0);
-    const int n[3] = {b.g.nx, b.g.ny, b.g.nz};
     int c[3];
-    float u[3], edge = 1.f;
-    bool out = false, cell = true;
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-    {
-        const float v = __fmaf_rn(f.M[3 * a], x, __fmaf_rn(f.M[3 * a + 1], y, __fmaf_rn(f.M[3 * a + 2], z, f.t[a])));
-        out = out || v < -e || v > (float)(n[a] - 1) + e;
-        // floor by rounding v - 1/2 at 1.5 2^23; a point that this rounds the
-        // other way lies on a cell boundary, which `edge` tells
-        const float r = (v - 0.5f) + 12582912.f;
-        c[a] = __float_as_int(r) - 0x4b400000;
-        u[a] = v - (r - 12582912.f);
-        edge = fminf(edge, fminf(u[a], 1.f - u[a]));
-        cell = cell && (unsigned)c[a] < (unsigned)(n[a] - 1);
-    }
-    if (out) return kOut32;
-    if (!cell || !(edge > e) || !(e < 0.25f)) return kUnsure32;
-    const float4* q = b.g.cell8 + 2 * (c[0] + (int64_t)n[0] * (c[1] + (int64_t)n[1] * c[2]));
+    float u[3], e;
+    const int at = place32(b.g, f, (float)X[0], (float)X[1], (float)X[2], c, u, e);
+    if (at != kInside32) return at;
+    const float4* q = b.g.cell8 + 2 * (c[0] + (int64_t)b.g.nx * (c[1] + (int64_t)b.g.ny * c[2]));
     const float4 p = __ldg(q), w = __ldg(q + 1);
     auto mix = [](float a0, float a1, float k) { return __fmaf_rn(k, a1 - a0, a0); };
     g = mix(mix(mix(p.x, p.y, u[0]), mix(p.z, p.w, u[0]), u[1]), mix(mix(w.x, w.y, u[0]), mix(w.z, w.w, u[0]), u[1]),
@@ -866,7 +830,7 @@ __device__ __noinline__ void measure_pass(const BeView& b, Shared& s)
     MinRec best{INFINITY, INT_MAX, -1};
     int nv = 0, na = 0;
     float least = INFINITY; // no gap below it is needed
-    Frame32 fr;
+    Place32 fr;
     if (BOUNDS)
     {
         frame32(b, s, fr);
@@ -886,7 +850,7 @@ __device__ __noinline__ void measure_pass(const BeView& b, Shared& s)
         {
             float g32, eps;
             const int k = gap32(b, fr, X, g32, eps);
-            if (k == kOut32) continue;
+            if (k == kOutside32) continue;
             if (k == kInside32)
             {
                 least = fminf(least, g32 + eps);

@@ -31,7 +31,7 @@
 // exactly nothing.  Dense grids keep one bit per cell that says whether the
 // interpolated gap can be <= 0 there (GridView::touch); a first pass places
 // every point in FP32 and lists those whose cell has the bit, or whose cell
-// FP32 cannot tell (TouchFrame), and only the listed points take the FP64
+// FP32 cannot tell (place32.cuh), and only the listed points take the FP64
 // transform, the gather and the law, shared out over all warps.  4096 poses of
 // a 7,680-point ring about a block's face, a quarter of them in contact: forces
 // and Jacobian 750 -> 281 us (one B200); bound by the latency of the few FP64
@@ -39,6 +39,7 @@
 #include <climits>
 
 #include "interp.cuh"
+#include "place32.cuh"
 
 namespace sdfo {
 namespace {
@@ -218,18 +219,9 @@ __device__ __forceinline__ int point_state(const GridView& g, const float* __res
     return 2;
 }
 
-// A pose's map from quadrature points to grid index coordinates in FP32:
-// f = M x + t with M = R_B^T R_A / h, t = (R_B^T (r_A - r_B) - bmin) / h - 1/2.
-// M, t and three fused steps are each rounded to 2^-24 of at most
-// |M|max |x|_1 + |t|max, so f is within e0 + e1 |x|_1 of the FP64 value.
-struct TouchFrame
-{
-    float M[9], t[3], e0, e1;
-};
-
 // Entry `q` of M (0..8) or t (9..11), for threads 0..11.
 __device__ __forceinline__ void set_touch_entry(const GridView& g, const sdfo_body_state& sA,
-                                                const sdfo_body_state& sB, const v3& tl, int q, TouchFrame& f)
+                                                const sdfo_body_state& sB, const v3& tl, int q, Place32& f)
 {
     if (q < 9)
     {
@@ -243,15 +235,6 @@ __device__ __forceinline__ void set_touch_entry(const GridView& g, const sdfo_bo
     }
 }
 
-__device__ __forceinline__ void set_touch_margin(TouchFrame& f)
-{
-    float m = 0.f;
-#pragma unroll
-    for (int q = 0; q < 9; ++q) m = fmaxf(m, fabsf(f.M[q]));
-    f.e1 = m * 0x1p-21f;
-    f.e0 = fmaxf(fabsf(f.t[0]), fmaxf(fabsf(f.t[1]), fabsf(f.t[2]))) * 0x1p-21f + 0x1p-28f;
-}
-
 enum : int
 {
     kOutside = 0, // certainly outside the grid
@@ -259,31 +242,15 @@ enum : int
     kMayTouch = 2 // anything else: the FP64 path decides
 };
 
-__device__ __forceinline__ int touch_status(const GridView& g, const uint32_t* __restrict__ bits, const TouchFrame& f,
+__device__ __forceinline__ int touch_status(const GridView& g, const uint32_t* __restrict__ bits, const Place32& f,
                                             float x, float y, float z)
 {
-    const float e = __fmaf_rn(fabsf(x) + fabsf(y) + fabsf(z), f.e1, f.e0);
-    const int n[3] = {g.nx, g.ny, g.nz};
     int c[3];
-    bool out = false;
-    float edge = 1.f; // distance to the nearest cell boundary
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-    {
-        const float v = __fmaf_rn(f.M[3 * a], x, __fmaf_rn(f.M[3 * a + 1], y, __fmaf_rn(f.M[3 * a + 2], z, f.t[a])));
-        out = out || v < -e || v > (float)(n[a] - 1) + e;
-        // floor by rounding v - 1/2 at 1.5 2^23 (|v| < 2^20; a point that this
-        // rounds the other way lies on a boundary)
-        const float r = (v - 0.5f) + 12582912.f;
-        c[a] = __float_as_int(r) - 0x4b400000;
-        const float u = v - (r - 12582912.f);
-        edge = fminf(edge, fminf(u, 1.f - u));
-    }
-    const bool cell = !out && edge > e && e < 0.25f && (unsigned)c[0] < (unsigned)(n[0] - 1) &&
-                      (unsigned)c[1] < (unsigned)(n[1] - 1) && (unsigned)c[2] < (unsigned)(n[2] - 1);
-    const int i = cell ? c[0] + n[0] * (c[1] + n[1] * c[2]) : 0;
+    float u[3], e;
+    const int at = place32(g, f, x, y, z, c, u, e);
+    const int i = at == kInside32 ? c[0] + g.nx * (c[1] + g.ny * c[2]) : 0;
     const uint32_t w = __ldg(bits + (i >> 5)); // no branch about it: loads of several points overlap
-    return out ? kOutside : cell && !((w >> (i & 31)) & 1u) ? kClear : kMayTouch;
+    return at == kOutside32 ? kOutside : at == kInside32 && !((w >> (i & 31)) & 1u) ? kClear : kMayTouch;
 }
 
 // Column j of the point's d(f, x f)/d(dx, dtheta), weighted by w.
@@ -409,7 +376,7 @@ __global__ void __launch_bounds__(T, T == kFewThreads ? 1 : JAC ? SDFO_CONTACT_J
     __shared__ int s_list[LIST ? kJacSpan : 1];
     __shared__ int s_act[TOUCH && JAC ? kJacSpan : 1];
     __shared__ int s_acnt[kWarps];
-    __shared__ TouchFrame s_touch;
+    __shared__ Place32 s_touch;
     __shared__ int s_wcnt[kWarps];
     __shared__ unsigned s_mask[EXT ? kMaxCullLeaves / 32 : 1];
     __shared__ double s_box[6];
@@ -438,13 +405,15 @@ __global__ void __launch_bounds__(T, T == kFewThreads ? 1 : JAC ? SDFO_CONTACT_J
     f.vB = V(sB.v[0], sB.v[1], sB.v[2]);
     f.wB = V(sB.w[0], sB.w[1], sB.w[2]);
     f.tl = mulT(sB.R, f.rA - f.rB); // R_B^T (r_A - r_B)
-    TouchFrame tf;
+    Place32 tf;
     if (TOUCH)
     {
         set_touch_entry(g, sA, sB, f.tl, (int)threadIdx.x, s_touch);
         __syncthreads();
         tf = s_touch;
-        set_touch_margin(tf);
+        tf.set_margin(fmax((fabs(f.tl.x) + fabs(g.bmin[0])) * g.ivoxel[0],
+                           fmax((fabs(f.tl.y) + fabs(g.bmin[1])) * g.ivoxel[1],
+                                (fabs(f.tl.z) + fabs(g.bmin[2])) * g.ivoxel[2])));
     }
 
     // broad phase: AABB_BVH.query(bmin_local, bmax_local) (bvh.py:62-80)
