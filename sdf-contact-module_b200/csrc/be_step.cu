@@ -280,27 +280,7 @@ __device__ __forceinline__ void frame32(const BeView& b, const Shared& s, Place3
         f.t[a] = (float)((s.tl[a] - b.g.bmin[a]) * b.g.ivoxel[a] - 0.5);
         far = fmax(far, (fabs(s.tl[a]) + fabs(b.g.bmin[a])) * b.g.ivoxel[a]);
     }
-    f.set_margin(far);
-}
-
-// The gap at X from the cell's FP32 corner record.  A coordinate off by e
-// moves the interpolant by at most e times the corners' spread per axis; the
-// corners and the interpolation are rounded to less than 2^-20 of the largest.
-__device__ __forceinline__ int gap32(const BeView& b, const Place32& f, const double X[3], float& g, float& eps)
-{
-    int c[3];
-    float u[3], e;
-    const int at = place32(b.g, f, (float)X[0], (float)X[1], (float)X[2], c, u, e);
-    if (at != kInside32) return at;
-    const float4* q = b.g.cell8 + 2 * (c[0] + (int64_t)b.g.nx * (c[1] + (int64_t)b.g.ny * c[2]));
-    const float4 p = __ldg(q), w = __ldg(q + 1);
-    auto mix = [](float a0, float a1, float k) { return __fmaf_rn(k, a1 - a0, a0); };
-    g = mix(mix(mix(p.x, p.y, u[0]), mix(p.z, p.w, u[0]), u[1]), mix(mix(w.x, w.y, u[0]), mix(w.z, w.w, u[0]), u[1]),
-            u[2]);
-    const float lo = fminf(fminf(fminf(p.x, p.y), fminf(p.z, p.w)), fminf(fminf(w.x, w.y), fminf(w.z, w.w)));
-    const float hi = fmaxf(fmaxf(fmaxf(p.x, p.y), fmaxf(p.z, p.w)), fmaxf(fmaxf(w.x, w.y), fmaxf(w.z, w.w)));
-    eps = __fmaf_rn(4.f * e, hi - lo, 0x1p-20f * fmaxf(fabsf(lo), fabsf(hi)));
-    return fabsf(g) < INFINITY && eps < INFINITY ? kInside32 : kUnsure32;
+    f.set_margin((float)far);
 }
 
 // R_sdf = R_B^T R_A, t_sdf = R_B^T (r_A - r_B) of a pose (contacts_sdf.py:
@@ -836,7 +816,10 @@ __device__ __noinline__ void measure_pass(const BeView& b, Shared& s)
         frame32(b, s, fr);
         double X[3], w;
         float g, eps;
-        if (s.mi >= 0 && point_at(b, s, s.mi, X, w) && gap32(b, fr, X, g, eps) == kInside32) least = g + eps;
+        bool out;
+        if (s.mi >= 0 && point_at(b, s, s.mi, X, w) &&
+            gap32(b.g, fr, (float)X[0], (float)X[1], (float)X[2], g, eps, out))
+            least = g + eps;
     }
     // ties of the minimum go to the first kept point; the list index orders
     // kept points as their positions among the kept points do, so it serves
@@ -849,9 +832,8 @@ __device__ __noinline__ void measure_pass(const BeView& b, Shared& s)
         if (BOUNDS)
         {
             float g32, eps;
-            const int k = gap32(b, fr, X, g32, eps);
-            if (k == kOutside32) continue;
-            if (k == kInside32)
+            bool out;
+            if (gap32(b.g, fr, (float)X[0], (float)X[1], (float)X[2], g32, eps, out))
             {
                 least = fminf(least, g32 + eps);
                 const bool below = g32 + eps < 0.f; // certainly active
@@ -862,6 +844,8 @@ __device__ __noinline__ void measure_pass(const BeView& b, Shared& s)
                     continue;
                 }
             }
+            else if (out)
+                continue;
         }
         to_sdf(s, X, Y);
         double g, gr[3];

@@ -50,9 +50,13 @@ namespace {
 // Jacobian: 299 us against 388).
 constexpr int kContactThreads = 256;
 constexpr int kFewThreads = 512;
-// Points are listed by spans of kJacSpan, per warp (a warp meets at most its
-// share of a span); then all warps share the span's list.
+// Points are listed by spans of kJacSpan; then all warps share the span's list.
 constexpr int kJacSpan = 4096;
+// With touch bits, 32 consecutive points go to list (their number) mod kRows, 32
+// consecutive entries of the span's list to partial sum (their number) mod
+// kRows: a pose's sums run in one order whatever the threads per pose, so its
+// forces do not depend on the other poses of the call.
+constexpr int kRows = kFewThreads / 32;
 // Points per thread in flight in the pass over the touch bits.
 constexpr int kAhead = 4;
 
@@ -219,10 +223,12 @@ __device__ __forceinline__ int point_state(const GridView& g, const float* __res
     return 2;
 }
 
-// Entry `q` of M (0..8) or t (9..11), for threads 0..11.
-__device__ __forceinline__ void set_touch_entry(const GridView& g, const sdfo_body_state& sA,
+// Entry `q` of M (0..8), of t (9..11), or set_margin's argument (12, in e0), for
+// threads 0..12.
+__device__ __forceinline__ void set_place_entry(const GridView& g, const sdfo_body_state& sA,
                                                 const sdfo_body_state& sB, const v3& tl, int q, Place32& f)
 {
+    const double t[3] = {tl.x, tl.y, tl.z};
     if (q < 9)
     {
         const int a = q / 3, b = q % 3;
@@ -232,6 +238,13 @@ __device__ __forceinline__ void set_touch_entry(const GridView& g, const sdfo_bo
     {
         const int a = q - 9;
         f.t[a] = (float)(((a == 0 ? tl.x : a == 1 ? tl.y : tl.z) - g.bmin[a]) * g.ivoxel[a] - 0.5);
+    }
+    else if (q == 12)
+    {
+        double far = 0.0;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) far = fmax(far, (fabs(t[a]) + fabs(g.bmin[a])) * g.ivoxel[a]);
+        f.e0 = (float)far;
     }
 }
 
@@ -247,10 +260,11 @@ __device__ __forceinline__ int touch_status(const GridView& g, const uint32_t* _
 {
     int c[3];
     float u[3], e;
-    const int at = place32(g, f, x, y, z, c, u, e);
-    const int i = at == kInside32 ? c[0] + g.nx * (c[1] + g.ny * c[2]) : 0;
+    bool out;
+    const bool cell = place32(g, f, x, y, z, c, u, e, out);
+    const int i = cell ? c[0] + g.nx * (c[1] + g.ny * c[2]) : 0;
     const uint32_t w = __ldg(bits + (i >> 5)); // no branch about it: loads of several points overlap
-    return at == kOutside32 ? kOutside : at == kInside32 && !((w >> (i & 31)) & 1u) ? kClear : kMayTouch;
+    return out ? kOutside : cell && !((w >> (i & 31)) & 1u) ? kClear : kMayTouch;
 }
 
 // Column j of the point's d(f, x f)/d(dx, dtheta), weighted by w.
@@ -355,48 +369,20 @@ __device__ __forceinline__ int warp_isum(int v)
     return v;
 }
 
-// EXT: the culled / measuring variant (ContactCull, measures); without it
-// every point is evaluated and no measure is produced.
-// TOUCH: `bits` are the mode's touch bits of a dense grid.  The first pass lists
-// the points that may touch (with JAC alone: the points in contact), the second
-// evaluates the list.
-template <int MODE, bool SPARSE, int BD, bool JAC, bool EXT, bool TOUCH, int T>
-__global__ void __launch_bounds__(T, T == kFewThreads ? 1 : JAC ? SDFO_CONTACT_JAC_MIN_BLOCKS : SDFO_CONTACT_MIN_BLOCKS)
-    k_contact(GridView g, const float* __restrict__ qx, const float* __restrict__ qw, int nq,
-              const sdfo_body_state* __restrict__ poses, const sdfo_body_state* __restrict__ body_b,
-              sdfo_contact_params prm, double* __restrict__ ft, double* __restrict__ jac, ContactCull cull,
-              sdfo_contact_measure* __restrict__ meas, const uint32_t* __restrict__ bits)
+// The pose's body states into shared memory, 18 doubles each, one per thread.
+__device__ __forceinline__ void load_states(const sdfo_body_state* pose, const sdfo_body_state* body_b,
+                                            sdfo_body_state& sA, sdfo_body_state& sB)
 {
-    constexpr int kWarps = T / 32, kJacPerWarp = kJacSpan / kWarps;
-    const int pose = blockIdx.x;
-    __shared__ sdfo_body_state sA, sB;
-    __shared__ double red[kWarps][6];
-    __shared__ double sjac[JAC ? kWarps : 1][JAC ? 36 : 1];
-    constexpr bool LIST = JAC || TOUCH;
-    __shared__ int s_list[LIST ? kJacSpan : 1];
-    __shared__ int s_act[TOUCH && JAC ? kJacSpan : 1];
-    __shared__ int s_acnt[kWarps];
-    __shared__ Place32 s_touch;
-    __shared__ int s_wcnt[kWarps];
-    __shared__ unsigned s_mask[EXT ? kMaxCullLeaves / 32 : 1];
-    __shared__ double s_box[6];
-    __shared__ int s_full;
-    __shared__ MinRec s_min[EXT ? kWarps : 1];
-    __shared__ int s_cnt[EXT ? kWarps : 1][2];
-    __shared__ int s_prefix;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    {
-        // 18 doubles each, one per thread
-        static_assert(sizeof(sdfo_body_state) == 18 * sizeof(double), "a body state is 18 doubles");
-        const int q = (int)threadIdx.x;
-        if (q < 18)
-            reinterpret_cast<double*>(&sA)[q] = __ldg(reinterpret_cast<const double*>(poses + pose) + q);
-        else if (q < 36)
-            reinterpret_cast<double*>(&sB)[q - 18] = __ldg(reinterpret_cast<const double*>(body_b) + q - 18);
-    }
-    if (JAC)
-        for (int t = lane; t < 36; t += 32) sjac[warp][t] = 0.0;
-    __syncthreads();
+    static_assert(sizeof(sdfo_body_state) == 18 * sizeof(double), "a body state is 18 doubles");
+    const int q = (int)threadIdx.x;
+    if (q < 18)
+        reinterpret_cast<double*>(&sA)[q] = __ldg(reinterpret_cast<const double*>(pose) + q);
+    else if (q < 36)
+        reinterpret_cast<double*>(&sB)[q - 18] = __ldg(reinterpret_cast<const double*>(body_b) + q - 18);
+}
+
+__device__ __forceinline__ PoseFrame pose_frame(const sdfo_body_state& sA, const sdfo_body_state& sB)
+{
     PoseFrame f;
     f.rA = V(sA.r[0], sA.r[1], sA.r[2]);
     f.rB = V(sB.r[0], sB.r[1], sB.r[2]);
@@ -405,100 +391,321 @@ __global__ void __launch_bounds__(T, T == kFewThreads ? 1 : JAC ? SDFO_CONTACT_J
     f.vB = V(sB.v[0], sB.v[1], sB.v[2]);
     f.wB = V(sB.w[0], sB.w[1], sB.w[2]);
     f.tl = mulT(sB.R, f.rA - f.rB); // R_B^T (r_A - r_B)
+    return f;
+}
+
+// Broad phase: AABB_BVH.query(bmin_local, bmax_local) (bvh.py:62-80).
+struct BroadShared
+{
+    unsigned mask[kMaxCullLeaves / 32]; // leaves kept
+    double box[6];
+    int full;
+};
+
+// True: every point is kept (the mask is not set).  All threads call it.
+template <int T>
+__device__ __forceinline__ bool broad_phase(const ContactCull& cull, const sdfo_body_state& sA, const PoseFrame& f,
+                                            BroadShared& s)
+{
+    if (!cull.enabled) return true;
+    if (threadIdx.x == 0)
+    {
+        const v3 lo = mulT(sA.R, V(cull.bmin[0], cull.bmin[1], cull.bmin[2]) - f.rA);
+        const v3 hi = mulT(sA.R, V(cull.bmax[0], cull.bmax[1], cull.bmax[2]) - f.rA);
+        s.box[0] = lo.x - cull.box_margin;
+        s.box[1] = lo.y - cull.box_margin;
+        s.box[2] = lo.z - cull.box_margin;
+        s.box[3] = hi.x + cull.box_margin;
+        s.box[4] = hi.y + cull.box_margin;
+        s.box[5] = hi.z + cull.box_margin;
+        bool enc = true;
+        for (int a = 0; a < 3; ++a) enc = enc && s.box[a] <= cull.root[a] && s.box[3 + a] >= cull.root[3 + a];
+        s.full = enc ? 1 : 0;
+    }
+    for (int w = threadIdx.x; w < (cull.nleaves + 31) / 32; w += T) s.mask[w] = 0u;
+    __syncthreads();
+    if (s.full != 0) return true;
+    bool any = false;
+    for (int l = threadIdx.x; l < cull.nleaves; l += T)
+    {
+        const double* b = cull.leaf_box + 6 * (int64_t)l;
+        const bool skip = b[3] < s.box[0] || b[4] < s.box[1] || b[5] < s.box[2] || b[0] > s.box[3] ||
+                          b[1] > s.box[4] || b[2] > s.box[5];
+        if (!skip)
+        {
+            atomicOr(&s.mask[l >> 5], 1u << (l & 31));
+            any = true;
+        }
+    }
+    return __syncthreads_or(any) == 0; // no leaf: every point (contacts_sdf.py:268-269)
+}
+
+// What a thread has measured.
+struct Measured
+{
+    MinRec best{INFINITY, INT_MAX, -1};
+    int nvalid = 0, nactive = 0;
+    __device__ __forceinline__ void point(const ContactCull& cull, bool full, int i, double gap)
+    {
+        ++nvalid;
+        if (gap < 0.0) ++nactive;
+        const MinRec r{gap, full ? (cull.porig ? __ldg(cull.porig + i) : i) : i, i};
+        if (less_rec(r, best)) best = r;
+    }
+};
+
+template <int WARPS>
+struct MeasureShared
+{
+    MinRec min[WARPS];
+    int cnt[WARPS][2];
+    int prefix;
+};
+
+// measure_pair's result from all threads' (contacts_sdf.py:171-214).
+template <int MODE, bool SPARSE, int BD, int T>
+__device__ __forceinline__ void write_measure(const GridView& g, const float* __restrict__ qx,
+                                              const sdfo_body_state& sA, const sdfo_body_state& sB, const PoseFrame& f,
+                                              const ContactCull& cull, bool full, const BroadShared& broad,
+                                              MeasureShared<T / 32>& s, const Measured& mine,
+                                              sdfo_contact_measure* __restrict__ out_at)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    {
+        const MinRec r = warp_min(mine.best);
+        const int nv = warp_isum(mine.nvalid), na = warp_isum(mine.nactive);
+        if (lane == 0)
+        {
+            s.min[warp] = r;
+            s.cnt[warp][0] = nv;
+            s.cnt[warp][1] = na;
+        }
+        if (threadIdx.x == 0) s.prefix = 0;
+    }
+    __syncthreads();
+    MinRec b = s.min[0];
+    int nv = s.cnt[0][0], na = s.cnt[0][1];
+#pragma unroll
+    for (int w = 1; w < T / 32; ++w)
+    {
+        if (less_rec(s.min[w], b)) b = s.min[w];
+        nv += s.cnt[w][0];
+        na += s.cnt[w][1];
+    }
+    // position of the minimum in the broad phase's point list: the points of
+    // the kept leaves before its own
+    if (nv > 0 && !full)
+    {
+        const int lb = __ldg(cull.pleaf + b.i);
+        int part = 0;
+        for (int l = threadIdx.x; l < lb; l += T)
+            if ((broad.mask[l >> 5] >> (l & 31)) & 1u) part += __ldg(cull.leaf_start + l + 1) - __ldg(cull.leaf_start + l);
+        part = warp_isum(part);
+        if (lane == 0 && part) atomicAdd(&s.prefix, part);
+        __syncthreads();
+    }
+    if (threadIdx.x != 0) return;
+    sdfo_contact_measure out;
+    out.reserved0 = 0;
+    out.active_count = na;
+    out.valid_count = nv;
+    if (nv == 0)
+    {
+        out.gap = INFINITY;
+        out.penetration = 0.0;
+        out.normal_velocity = 0.0;
+        out.min_point_index = -1;
+    }
+    else
+    {
+        out.gap = b.gap;
+        out.penetration = b.gap < 0.0 ? -b.gap : 0.0;
+        out.min_point_index = full ? b.key : s.prefix + (b.i - __ldg(cull.leaf_start + __ldg(cull.pleaf + b.i)));
+        // normal relative velocity at the minimum (contacts_sdf.py:199-211)
+        const v3 X = V(__ldg(qx + 3 * b.i), __ldg(qx + 3 * b.i + 1), __ldg(qx + 3 * b.i + 2));
+        const v3 off = mul(sA.R, X);
+        const v3 Yv = mulT(sB.R, off) + f.tl;
+        const double Y[3] = {Yv.x, Yv.y, Yv.z};
+        float gapf;
+        v3 gl;
+        double Hl[6];
+        sample<MODE, SPARSE, BD, false>(g, Y, gapf, gl, Hl);
+        const double gn = sqrt(dot(gl, gl));
+        const v3 un = gn > 1e-30 ? (1.0 / gn) * gl : V(0.0, 0.0, 1.0);
+        v3 nw = mul(sB.R, un);
+        const double nn = sqrt(dot(nw, nw));
+        if (nn > 1e-30) nw = (1.0 / nn) * nw;
+        const v3 xw = f.rA + off;
+        const v3 uA = f.vA + cross(f.wA, off);
+        const v3 uB = f.vB + cross(f.wB, xw - f.rB);
+        out.normal_velocity = dot(uA - uB, nw);
+    }
+    *out_at = out;
+}
+
+// N lists of kJacSpan / N entries at most, taken one after the other: their
+// lengths' inclusive prefix, lane by lane, and from it the place of entry e.  All
+// lanes call both.  (Held in registers, sixteen lengths would spill in the loops
+// of the force law.)
+template <int N>
+struct Lists
+{
+    int pre, total;
+    __device__ __forceinline__ explicit Lists(const int* lengths)
+    {
+        const int lane = (int)(threadIdx.x & 31);
+        pre = lane < N ? lengths[lane] : 0;
+#pragma unroll
+        for (int o = 1; o < N; o *= 2)
+        {
+            const int q = __shfl_up_sync(0xffffffffu, pre, o);
+            if (lane >= o) pre += q;
+        }
+        total = __shfl_sync(0xffffffffu, pre, N - 1);
+    }
+    __device__ __forceinline__ int place(int e) const
+    {
+        int src = 0;
+#pragma unroll
+        for (int o = N / 2; o > 0; o /= 2)
+            if (__shfl_sync(0xffffffffu, pre, src + o - 1) <= e) src += o;
+        const int before = __shfl_sync(0xffffffffu, pre, src > 0 ? src - 1 : 0);
+        return src * (kJacSpan / N) + e - (src > 0 ? before : 0);
+    }
+};
+
+// The Jacobian of the listed points in contact, into kLists partial sums.
+template <int MODE, bool SPARSE, int BD, bool TOUCH, int T>
+__device__ __forceinline__ void jacobian_pass(const GridView& g, const float* __restrict__ qx,
+                                              const float* __restrict__ qw, const sdfo_body_state& sA,
+                                              const sdfo_body_state& sB, const PoseFrame& f,
+                                              const sdfo_contact_params& prm, double narrow, const int* list,
+                                              const int* lengths, double (*sums)[36])
+{
+    constexpr int kWarps = T / 32, kLists = TOUCH ? kRows : kWarps;
+    const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
+    const Lists<kLists> lists(lengths);
+    auto add_column = [&](const double col[6], int row, int j) {
+#pragma unroll
+        for (int r = 0; r < 6; ++r)
+        {
+            const double sum = warp_sum(col[r]);
+            if (lane == 0) sums[row][6 * r + j] += sum;
+        }
+    };
+    auto in_contact = [&](int e, int at, PointState& st) {
+        double gap = 0.0;
+        return e < lists.total && point_state<MODE, SPARSE, BD, true>(g, qx, qw, list[at], sA, sB, f, prm, narrow, false,
+                                                                      st, gap) == 2;
+    };
+    // one column of 32 points in contact at a time
+    for (int k = warp; 32 * (k / 6) < lists.total; k += kWarps) // warp-uniform
+    {
+        const int e = 32 * (k / 6) + lane, at = lists.place(e);
+        double col[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        PointState st;
+        if (in_contact(e, at, st)) jacobian_column(st, sB, f, prm, k % 6, col);
+        add_column(col, k % kLists, k % 6);
+    }
+}
+
+// The sum of N values `stride` apart, by halves.
+template <int N>
+__device__ __forceinline__ double row_sum(const double* p, int stride)
+{
+    double v[N];
+#pragma unroll
+    for (int w = 0; w < N; ++w) v[w] = p[w * stride];
+#pragma unroll
+    for (int h = N / 2; h > 0; h /= 2)
+#pragma unroll
+        for (int w = 0; w < h; ++w) v[w] += v[w + h];
+    return v[0];
+}
+
+// EXT: the culled / measuring variant (ContactCull, measures); without it
+// every point is evaluated and no measure is produced.
+// TOUCH: `bits` are the mode's touch bits of a dense grid.  The first pass lists
+// the points that may touch (with JAC alone: the points in contact), the second
+// evaluates the list.
+template <int MODE, bool SPARSE, int BD, bool JAC, bool EXT, bool TOUCH, int T, int MB>
+__global__ void __launch_bounds__(T, MB)
+    k_contact(GridView g, const float* __restrict__ qx, const float* __restrict__ qw, int nq,
+              const sdfo_body_state* __restrict__ poses, const sdfo_body_state* __restrict__ body_b,
+              sdfo_contact_params prm, double* __restrict__ ft, double* __restrict__ jac,
+              ContactCull cull,
+              sdfo_contact_measure* __restrict__ meas, const uint32_t* __restrict__ bits)
+{
+    constexpr int kWarps = T / 32;
+    constexpr int kLists = TOUCH ? kRows : kWarps, kPerList = kJacSpan / kLists;
+    constexpr int kOwn = kLists / kWarps; // lists and sums w, w + kWarps, .. are warp w's
+    const int pose = blockIdx.x;
+    __shared__ sdfo_body_state sA, sB;
+    __shared__ double red[kLists][6];
+    __shared__ double sjac[JAC ? kLists : 1][36];
+    constexpr bool LIST = JAC || TOUCH;
+    __shared__ int s_list[LIST ? kJacSpan : 1];
+    __shared__ int s_act[TOUCH && JAC ? kJacSpan : 1];
+    __shared__ int s_acnt[kLists];
+    __shared__ Place32 s_touch;
+    __shared__ int s_wcnt[kLists];
+    __shared__ BroadShared s_broad;
+    __shared__ MeasureShared<kWarps> s_meas;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    load_states(poses + pose, body_b, sA, sB);
+    if (JAC)
+        for (int t = threadIdx.x; t < kLists * 36; t += T) (&sjac[0][0])[t] = 0.0;
+    if (TOUCH && threadIdx.x < kLists * 6) (&red[0][0])[threadIdx.x] = 0.0;
+    __syncthreads();
+    const PoseFrame f = pose_frame(sA, sB);
     Place32 tf;
     if (TOUCH)
     {
-        set_touch_entry(g, sA, sB, f.tl, (int)threadIdx.x, s_touch);
+        set_place_entry(g, sA, sB, f.tl, (int)threadIdx.x, s_touch);
         __syncthreads();
         tf = s_touch;
-        tf.set_margin(fmax((fabs(f.tl.x) + fabs(g.bmin[0])) * g.ivoxel[0],
-                           fmax((fabs(f.tl.y) + fabs(g.bmin[1])) * g.ivoxel[1],
-                                (fabs(f.tl.z) + fabs(g.bmin[2])) * g.ivoxel[2])));
+        tf.set_margin(s_touch.e0);
     }
 
-    // broad phase: AABB_BVH.query(bmin_local, bmax_local) (bvh.py:62-80)
-    bool full = true;
-    if (EXT && cull.enabled)
-    {
-        if (threadIdx.x == 0)
-        {
-            const v3 lo = mulT(sA.R, V(cull.bmin[0], cull.bmin[1], cull.bmin[2]) - f.rA);
-            const v3 hi = mulT(sA.R, V(cull.bmax[0], cull.bmax[1], cull.bmax[2]) - f.rA);
-            s_box[0] = lo.x - cull.box_margin;
-            s_box[1] = lo.y - cull.box_margin;
-            s_box[2] = lo.z - cull.box_margin;
-            s_box[3] = hi.x + cull.box_margin;
-            s_box[4] = hi.y + cull.box_margin;
-            s_box[5] = hi.z + cull.box_margin;
-            bool enc = true;
-            for (int a = 0; a < 3; ++a)
-                enc = enc && s_box[a] <= cull.root[a] && s_box[3 + a] >= cull.root[3 + a];
-            s_full = enc ? 1 : 0;
-        }
-        for (int w = threadIdx.x; w < (cull.nleaves + 31) / 32; w += T) s_mask[w] = 0u;
-        __syncthreads();
-        full = s_full != 0;
-        if (!full)
-        {
-            bool any = false;
-            for (int l = threadIdx.x; l < cull.nleaves; l += T)
-            {
-                const double* b = cull.leaf_box + 6 * (int64_t)l;
-                const bool skip = b[3] < s_box[0] || b[4] < s_box[1] || b[5] < s_box[2] || b[0] > s_box[3] ||
-                                  b[1] > s_box[4] || b[2] > s_box[5];
-                if (!skip)
-                {
-                    atomicOr(&s_mask[l >> 5], 1u << (l & 31));
-                    any = true;
-                }
-            }
-            full = __syncthreads_or(any) == 0; // no leaf: every point (contacts_sdf.py:268-269)
-        }
-    }
+    const bool full = EXT ? broad_phase<T>(cull, sA, f, s_broad) : true;
     const double narrow = EXT && cull.enabled ? cull.narrow_margin : -1.0;
     const bool want_force = ft != nullptr;
     const bool want_meas = EXT && meas != nullptr;
     double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    MinRec best{INFINITY, INT_MAX, -1};
-    int nvalid = 0, nactive = 0;
+    Measured seen;
 
     // whether the broad phase keeps point i
     auto kept = [&](int i) {
         if (!EXT || full) return true;
         const int l = __ldg(cull.pleaf + i);
-        return ((s_mask[l >> 5] >> (l & 31)) & 1u) != 0;
+        return ((s_broad.mask[l >> 5] >> (l & 31)) & 1u) != 0;
     };
-    auto measure_point = [&](int i, double gap) {
-        ++nvalid;
-        if (gap < 0.0) ++nactive;
-        const MinRec r{gap, full ? (cull.porig ? __ldg(cull.porig + i) : i) : i, i};
-        if (less_rec(r, best)) best = r;
-    };
-    auto add_force = [&](const PointState& st) {
+    auto add_force = [&](const PointState& st, double* sum) {
         const v3 tq = cross(st.off, st.fq);
-        acc[0] = fma(st.wq, st.fq.x, acc[0]);
-        acc[1] = fma(st.wq, st.fq.y, acc[1]);
-        acc[2] = fma(st.wq, st.fq.z, acc[2]);
-        acc[3] = fma(st.wq, tq.x, acc[3]);
-        acc[4] = fma(st.wq, tq.y, acc[4]);
-        acc[5] = fma(st.wq, tq.z, acc[5]);
+        sum[0] = fma(st.wq, st.fq.x, sum[0]);
+        sum[1] = fma(st.wq, st.fq.y, sum[1]);
+        sum[2] = fma(st.wq, st.fq.z, sum[2]);
+        sum[3] = fma(st.wq, tq.x, sum[3]);
+        sum[4] = fma(st.wq, tq.y, sum[4]);
+        sum[5] = fma(st.wq, tq.z, sum[5]);
     };
 
     // Spans of kJacSpan points (one span over all points when nothing is
     // listed).  First every point: by its touch bit, or by the forward law; each
     // warp lists its points, in point order, with no barrier.  Then the span's
-    // list is shared out: group k of 32 consecutive entries to warp k mod 8, so
+    // list, one list after the other, is shared out by groups of 32 entries, so
     // all warps carry the FP64 work, and the sums run in a fixed order (repeated
     // runs are bit-identical).  Block-uniform trip counts: the barriers and warp
     // reductions below see every thread.
     for (int s0 = 0; s0 < nq; s0 += LIST ? kJacSpan : nq)
     {
     const int s1 = LIST ? min(nq, s0 + kJacSpan) : nq;
-    int wcnt = 0; // this warp's listed points in the span (warp-uniform)
-    auto list_point = [&](bool listed, int i) {
+    int wcnt[kOwn] = {}; // listed points of the warp's lists (warp-uniform)
+    // appends the lanes' points to a list of which `count` are filled
+    auto append = [&](int* list, int& count, bool listed, int i) {
         const unsigned m = __ballot_sync(0xffffffffu, listed);
-        if (listed) s_list[warp * kJacPerWarp + wcnt + __popc(m & ((1u << lane) - 1u))] = i;
-        wcnt += __popc(m);
+        if (listed) list[count + __popc(m & ((1u << lane) - 1u))] = i;
+        count += __popc(m);
     };
     if constexpr (TOUCH)
     {
@@ -522,8 +729,9 @@ __global__ void __launch_bounds__(T, T == kFewThreads ? 1 : JAC ? SDFO_CONTACT_J
 #pragma unroll
             for (int u = 0; u < kAhead; ++u)
             {
-                if (want_meas && in[u] && status[u] == kClear) ++nvalid;
-                list_point(in[u] && status[u] == kMayTouch, i0 + u * T);
+                if (want_meas && in[u] && status[u] == kClear) ++seen.nvalid;
+                append(s_list + (warp + (u % kOwn) * kWarps) * kPerList, wcnt[u % kOwn], in[u] && status[u] == kMayTouch,
+                       i0 + u * T);
             }
         }
     }
@@ -539,116 +747,86 @@ __global__ void __launch_bounds__(T, T == kFewThreads ? 1 : JAC ? SDFO_CONTACT_J
                 double gap = 0.0;
                 const int status =
                     point_state<MODE, SPARSE, BD, false>(g, qx, qw, i, sA, sB, f, prm, narrow, want_meas, st, gap);
-                if (want_meas && status > 0) measure_point(i, gap);
+                if (want_meas && status > 0) seen.point(cull, full, i, gap);
                 act = status == 2 && want_force;
-                if (act) add_force(st);
+                if (act) add_force(st, acc);
             }
-            if (LIST) list_point(act, i);
+            if (LIST) append(s_list + warp * kPerList, wcnt[0], act, i);
         }
     }
     if (LIST)
     {
-        if (lane == 0) s_wcnt[warp] = wcnt;
+        if (lane == 0)
+#pragma unroll
+            for (int o = 0; o < kOwn; ++o) s_wcnt[warp + o * kWarps] = wcnt[o];
         __syncthreads();
-        // entry e of the warps' lists one after the other
-        auto entry = [&](const int* list, const int* cnt, int e) {
-            int rem = e, src = 0;
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w)
-            {
-                const int c = cnt[w];
-                if (src == w && rem >= c)
-                {
-                    rem -= c;
-                    ++src;
-                }
-            }
-            return list[src * kJacPerWarp + rem];
-        };
-        auto entries = [&](const int* cnt) {
-            int total = 0;
-#pragma unroll
-            for (int w = 0; w < kWarps; ++w) total += cnt[w];
-            return total;
-        };
         if constexpr (TOUCH)
         {
-            const int total = entries(s_wcnt);
-            int acnt = 0;
-            for (int k = warp; 32 * k < total; k += kWarps) // warp-uniform
+            const Lists<kLists> lists(s_wcnt);
+            if (lists.total == 0)
             {
-                const int e = 32 * k + lane;
-                bool act = false;
-                int idx = 0;
-                if (e < total)
-                {
-                    idx = entry(s_list, s_wcnt, e);
-                    PointState st;
-                    double gap = 0.0;
-                    const int status =
-                        point_state<MODE, SPARSE, BD, false>(g, qx, qw, idx, sA, sB, f, prm, narrow, want_meas, st, gap);
-                    if (want_meas && status > 0) measure_point(idx, gap);
-                    act = status == 2 && want_force;
-                    if (act) add_force(st);
-                }
-                if (JAC)
-                {
-                    const unsigned m = __ballot_sync(0xffffffffu, act);
-                    if (act) s_act[warp * kJacPerWarp + acnt + __popc(m & ((1u << lane) - 1u))] = idx;
-                    acnt += __popc(m);
-                }
-            }
-            if (JAC)
-            {
-                if (lane == 0) s_acnt[warp] = acnt;
                 __syncthreads();
+                continue;
             }
+#pragma unroll 1
+            for (int row = warp; row < kRows; row += kWarps) // warp-uniform
+            {
+                int acnt = 0;
+                double sum[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+                for (int k = row; 32 * k < lists.total; k += kRows)
+                {
+                    const int e = 32 * k + lane, at = lists.place(e);
+                    bool act = false;
+                    int idx = 0;
+                    if (e < lists.total)
+                    {
+                        idx = s_list[at];
+                        PointState st;
+                        double gap = 0.0;
+                        const int status = point_state<MODE, SPARSE, BD, false>(g, qx, qw, idx, sA, sB, f, prm, narrow,
+                                                                                want_meas, st, gap);
+                        if (want_meas && status > 0) seen.point(cull, full, idx, gap);
+                        act = status == 2 && want_force;
+                        if (act) add_force(st, sum);
+                    }
+                    if (JAC) append(s_act + row * kPerList, acnt, act, idx);
+                }
+                if (JAC && lane == 0) s_acnt[row] = acnt;
+                if (want_force && 32 * row < lists.total)
+                {
+#pragma unroll
+                    for (int q = 0; q < 6; ++q)
+                    {
+                        const double v = warp_sum(sum[q]);
+                        if (lane == 0) red[row][q] += v;
+                    }
+                }
+            }
+            if (JAC) __syncthreads();
         }
         if constexpr (JAC)
         {
-            // one column of the Jacobian of 32 points in contact at a time
-            const int* list = TOUCH ? s_act : s_list;
-            const int* cnt = TOUCH ? s_acnt : s_wcnt;
-            const int total = entries(cnt);
-            for (int k = warp; 32 * (k / 6) < total; k += kWarps) // warp-uniform
-            {
-                const int e = 32 * (k / 6) + lane, j = k % 6;
-                double col[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-                if (e < total)
-                {
-                    PointState st;
-                    double gap = 0.0;
-                    if (point_state<MODE, SPARSE, BD, true>(g, qx, qw, entry(list, cnt, e), sA, sB, f, prm, narrow,
-                                                            false, st, gap) == 2)
-                        jacobian_column(st, sB, f, prm, j, col);
-                }
-#pragma unroll
-                for (int r = 0; r < 6; ++r)
-                {
-                    const double sum = warp_sum(col[r]);
-                    if (lane == 0) sjac[warp][6 * r + j] += sum;
-                }
-            }
+            jacobian_pass<MODE, SPARSE, BD, TOUCH, T>(g, qx, qw, sA, sB, f, prm, narrow, TOUCH ? s_act : s_list,
+                                                      TOUCH ? s_acnt : s_wcnt, sjac);
         }
         __syncthreads(); // s_list and s_wcnt are rewritten by the next span
     }
     }
-    if (TOUCH && want_meas && __syncthreads_or(best.gap <= 0.0) == 0)
+    if (TOUCH && want_meas && __syncthreads_or(seen.best.gap <= 0.0) == 0)
     {
         // Clear of the surface: the least gap is not among the listed points
         // (elsewhere gaps are positive), so every point is measured.
-        best = MinRec{INFINITY, INT_MAX, -1};
-        nvalid = nactive = 0;
+        seen = Measured{};
         for (int i = threadIdx.x; i < nq; i += T)
             if (kept(i))
             {
                 PointState st;
                 double gap = 0.0;
                 if (point_state<MODE, SPARSE, BD, false>(g, qx, qw, i, sA, sB, f, prm, narrow, true, st, gap) > 0)
-                    measure_point(i, gap);
+                    seen.point(cull, full, i, gap);
             }
     }
-    if (want_force)
+    if (!TOUCH && want_force)
     {
 #pragma unroll
         for (int q = 0; q < 6; ++q)
@@ -657,92 +835,17 @@ __global__ void __launch_bounds__(T, T == kFewThreads ? 1 : JAC ? SDFO_CONTACT_J
             if (lane == 0) red[warp][q] = s;
         }
     }
-    if (want_meas)
-    {
-        const MinRec r = warp_min(best);
-        const int nv = warp_isum(nvalid), na = warp_isum(nactive);
-        if (lane == 0)
-        {
-            s_min[warp] = r;
-            s_cnt[warp][0] = nv;
-            s_cnt[warp][1] = na;
-        }
-        if (threadIdx.x == 0) s_prefix = 0;
-    }
     __syncthreads();
     if (want_force && threadIdx.x < 6)
     {
-        double s = 0.0;
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) s += red[w][threadIdx.x];
-        ft[6 * (int64_t)pose + threadIdx.x] = s;
+        ft[6 * (int64_t)pose + threadIdx.x] = row_sum<kLists>(&red[0][threadIdx.x], 6);
     }
     if (JAC && jac != nullptr && threadIdx.x < 36)
     {
-        double s = 0.0;
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) s += sjac[w][threadIdx.x];
-        jac[36 * (int64_t)pose + threadIdx.x] = s;
+        jac[36 * (int64_t)pose + threadIdx.x] = row_sum<kLists>(&sjac[0][threadIdx.x], 36);
     }
-    if (!want_meas) return;
-    MinRec b = s_min[0];
-    int nv = s_cnt[0][0], na = s_cnt[0][1];
-#pragma unroll
-    for (int w = 1; w < kWarps; ++w)
-    {
-        if (less_rec(s_min[w], b)) b = s_min[w];
-        nv += s_cnt[w][0];
-        na += s_cnt[w][1];
-    }
-    // position of the minimum in the broad phase's point list: the points of
-    // the kept leaves before its own
-    if (nv > 0 && !full)
-    {
-        const int lb = __ldg(cull.pleaf + b.i);
-        int part = 0;
-        for (int l = threadIdx.x; l < lb; l += T)
-            if ((s_mask[l >> 5] >> (l & 31)) & 1u) part += __ldg(cull.leaf_start + l + 1) - __ldg(cull.leaf_start + l);
-        part = warp_isum(part);
-        if (lane == 0 && part) atomicAdd(&s_prefix, part);
-        __syncthreads();
-    }
-    if (threadIdx.x != 0) return;
-    sdfo_contact_measure out;
-    out.reserved0 = 0;
-    out.active_count = na;
-    out.valid_count = nv;
-    if (nv == 0)
-    {
-        out.gap = INFINITY;
-        out.penetration = 0.0;
-        out.normal_velocity = 0.0;
-        out.min_point_index = -1;
-    }
-    else
-    {
-        out.gap = b.gap;
-        out.penetration = b.gap < 0.0 ? -b.gap : 0.0;
-        out.min_point_index = full ? b.key : s_prefix + (b.i - __ldg(cull.leaf_start + __ldg(cull.pleaf + b.i)));
-        // normal relative velocity at the minimum (contacts_sdf.py:199-211)
-        const v3 X = V(__ldg(qx + 3 * b.i), __ldg(qx + 3 * b.i + 1), __ldg(qx + 3 * b.i + 2));
-        const v3 off = mul(sA.R, X);
-        const v3 Yv = mulT(sB.R, off) + f.tl;
-        const double Y[3] = {Yv.x, Yv.y, Yv.z};
-        float gapf;
-        v3 gl;
-        double Hl[6];
-        sample<MODE, SPARSE, BD, false>(g, Y, gapf, gl, Hl);
-        const double gn = sqrt(dot(gl, gl));
-        const v3 un = gn > 1e-30 ? (1.0 / gn) * gl : V(0.0, 0.0, 1.0);
-        v3 nw = mul(sB.R, un);
-        const double nn = sqrt(dot(nw, nw));
-        if (nn > 1e-30) nw = (1.0 / nn) * nw;
-        const v3 xw = f.rA + off;
-        const v3 uA = f.vA + cross(f.wA, off);
-        const v3 uB = f.vB + cross(f.wB, xw - f.rB);
-        out.normal_velocity = dot(uA - uB, nw);
-    }
-    meas[pose] = out;
+    if (want_meas)
+        write_measure<MODE, SPARSE, BD, T>(g, qx, sA, sB, f, cull, full, s_broad, s_meas, seen, meas + pose);
 }
 
 struct ContactLaunch
@@ -760,29 +863,30 @@ struct ContactLaunch
     sdfo_contact_measure* meas;
 };
 
-template <int MODE, bool SPARSE, int BD, bool EXT, bool TOUCH, int T>
+template <int MODE, bool SPARSE, int BD, bool EXT, bool TOUCH, int T, int MB, int JAC_MB>
 void launch5(const GridView& v, const ContactLaunch& c, const uint32_t* bits, cudaStream_t s)
 {
     if (c.jac)
-        k_contact<MODE, SPARSE, BD, true, EXT, TOUCH, T><<<c.np, T, 0, s>>>(
+        k_contact<MODE, SPARSE, BD, true, EXT, TOUCH, T, JAC_MB><<<c.np, T, 0, s>>>(
             v, c.qx, c.qw, c.nq, c.pa, c.pb, c.prm, c.ft, c.jac, c.cull, c.meas, bits);
     else
-        k_contact<MODE, SPARSE, BD, false, EXT, TOUCH, T><<<c.np, T, 0, s>>>(
+        k_contact<MODE, SPARSE, BD, false, EXT, TOUCH, T, MB><<<c.np, T, 0, s>>>(
             v, c.qx, c.qw, c.nq, c.pa, c.pb, c.prm, c.ft, c.jac, c.cull, c.meas, bits);
 }
 
 template <int MODE, bool SPARSE, int BD, bool EXT, bool TOUCH>
 void launch4(const GridView& v, const ContactLaunch& c, const uint32_t* bits, cudaStream_t s)
 {
+    constexpr int MB = SDFO_CONTACT_MIN_BLOCKS, JAC_MB = SDFO_CONTACT_JAC_MIN_BLOCKS;
     if constexpr (TOUCH)
     {
         if (c.np <= current_sm_count())
         {
-            launch5<MODE, SPARSE, BD, EXT, TOUCH, kFewThreads>(v, c, bits, s);
+            launch5<MODE, SPARSE, BD, EXT, TOUCH, kFewThreads, 1, 1>(v, c, bits, s);
             return;
         }
     }
-    launch5<MODE, SPARSE, BD, EXT, TOUCH, kContactThreads>(v, c, bits, s);
+    launch5<MODE, SPARSE, BD, EXT, TOUCH, kContactThreads, MB, JAC_MB>(v, c, bits, s);
 }
 
 template <int MODE, bool SPARSE, int BD, bool TOUCH>
