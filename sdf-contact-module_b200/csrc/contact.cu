@@ -57,6 +57,11 @@ constexpr int kJacSpan = 4096;
 // kRows: a pose's sums run in one order whatever the threads per pose, so its
 // forces do not depend on the other poses of the call.
 constexpr int kRows = kFewThreads / 32;
+// Groups of 32 points in contact up to which the Jacobian's columns are shared out
+// over the warps, every column evaluating its points anew.  4,096 poses in light
+// contact (about four groups): 613 us with the columns shared out up to here, 766
+// up to eight groups; in deep contact shared-out columns took 6.1 ms against 5.0.
+constexpr int kSplitGroups = 4;
 // Points per thread in flight in the pass over the touch bits.
 constexpr int kAhead = 4;
 
@@ -325,12 +330,14 @@ __device__ __forceinline__ void jacobian_column(const PointState& st, const sdfo
 // a small fraction) are listed and evaluated again with the interpolant's
 // Hessian for the six Jacobian columns; with touch bits all of that runs on
 // the listed points alone.
-// Resident CTAs per SM asked of the register allocator (256 threads each).
+// Resident CTAs per SM asked of the register allocator (256 threads each).  With
+// the Jacobian two, without spills: at three, points in deep contact, evaluated
+// for all six columns, ran 0.61 (sparse Tricubic) to 0.90 times as fast.
 #ifndef SDFO_CONTACT_MIN_BLOCKS
 #define SDFO_CONTACT_MIN_BLOCKS 3
 #endif
 #ifndef SDFO_CONTACT_JAC_MIN_BLOCKS
-#define SDFO_CONTACT_JAC_MIN_BLOCKS 3
+#define SDFO_CONTACT_JAC_MIN_BLOCKS 2
 #endif
 
 // Lexicographic (gap, key) minimum for measure_pair's argmin: the reference
@@ -598,14 +605,32 @@ __device__ __forceinline__ void jacobian_pass(const GridView& g, const float* __
         return e < lists.total && point_state<MODE, SPARSE, BD, true>(g, qx, qw, list[at], sA, sB, f, prm, narrow, false,
                                                                       st, gap) == 2;
     };
-    // one column of 32 points in contact at a time
-    for (int k = warp; 32 * (k / 6) < lists.total; k += kWarps) // warp-uniform
+    if (TOUCH && lists.total <= 32 * kSplitGroups)
     {
-        const int e = 32 * (k / 6) + lane, at = lists.place(e);
-        double col[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        // few points in contact: one column of 32 points at a time, so that more
+        // warps have work
+        for (int k = warp; 32 * (k / 6) < lists.total; k += kWarps) // warp-uniform
+        {
+            const int e = 32 * (k / 6) + lane, at = lists.place(e);
+            double col[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            PointState st;
+            if (in_contact(e, at, st)) jacobian_column(st, sB, f, prm, k % 6, col);
+            add_column(col, k % kLists, k % 6);
+        }
+        return;
+    }
+    for (int k = warp; 32 * k < lists.total; k += kWarps) // warp-uniform
+    {
+        const int e = 32 * k + lane, at = lists.place(e);
         PointState st;
-        if (in_contact(e, at, st)) jacobian_column(st, sB, f, prm, k % 6, col);
-        add_column(col, k % kLists, k % 6);
+        const bool mine = in_contact(e, at, st);
+#pragma unroll 1
+        for (int j = 0; j < 6; ++j)
+        {
+            double col[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            if (mine) jacobian_column(st, sB, f, prm, j, col);
+            add_column(col, k % kLists, j);
+        }
     }
 }
 
@@ -885,6 +910,15 @@ void launch4(const GridView& v, const ContactLaunch& c, const uint32_t* bits, cu
             launch5<MODE, SPARSE, BD, EXT, TOUCH, kFewThreads, 1, 1>(v, c, bits, s);
             return;
         }
+        // Trilinear Jacobians with touch bits gain by a third CTA where there are
+        // poses for it: 4,096 poses, a quarter in light contact, 321 us against
+        // 301; 149 poses in deep contact lose by it, 448 us against 514.
+        if constexpr (MODE == SDFO_TRILINEAR)
+            if (c.jac && c.np > 2 * current_sm_count())
+            {
+                launch5<MODE, SPARSE, BD, EXT, TOUCH, kContactThreads, MB, 3>(v, c, bits, s);
+                return;
+            }
     }
     launch5<MODE, SPARSE, BD, EXT, TOUCH, kContactThreads, MB, JAC_MB>(v, c, bits, s);
 }
