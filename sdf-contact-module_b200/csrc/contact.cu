@@ -873,6 +873,115 @@ __global__ void __launch_bounds__(T, MB)
         write_measure<MODE, SPARSE, BD, T>(g, qx, sA, sB, f, cull, full, s_broad, s_meas, seen, meas + pose);
 }
 
+// How a measure alone (no forces) meets its points.
+enum : int
+{
+    kEveryPoint = 0, // FP64 for each
+    kByBounds = 1,   // dense Trilinear: FP64 where FP32 bounds of the gap leave it open
+    kByTouch = 2     // dense Tricubic: FP64 where the touch bits leave it open; if no
+                     // gap is <= 0, for every point
+};
+
+// The least value of the warp's lanes (FP32 as ordered integers).
+__device__ __forceinline__ float warp_least(float v)
+{
+    const int b = __float_as_int(v);
+    const int m = __reduce_min_sync(0xffffffffu, b ^ ((b >> 31) & 0x7fffffff));
+    return __int_as_float(m ^ ((m >> 31) & 0x7fffffff));
+}
+
+// measure_pair of every pose, without the forces (one CTA per pose).  Bound by
+// the gather of every point and, for kEveryPoint, its FP64 transform.  kByBounds
+// reads the cell record that the FP64 path would read, in FP32 alone, and takes
+// the FP64 path only for points that may be the least (a warp shares the least
+// upper bound met) or whose sign is open; so every point that attains the least
+// gap is sampled, and gap, index and counts are those of sampling all.  4,096
+// poses of a 7,680-point ring about a block, clear of it / in light / in deep
+// contact, in the force kernel by touch bits and here (us): Trilinear 505 / 412 /
+// 669 and 289 / 309 / 283; Tricubic 594 / 310 / 760 and 477 / 271 / 445.
+template <int MODE, bool SPARSE, int BD, int HOW, int T, int MB>
+__global__ void __launch_bounds__(T, MB)
+    k_measure(GridView g, const float* __restrict__ qx, int nq, const sdfo_body_state* __restrict__ poses,
+              const sdfo_body_state* __restrict__ body_b, ContactCull cull, sdfo_contact_measure* __restrict__ meas,
+              const uint32_t* __restrict__ bits)
+{
+    const int pose = blockIdx.x;
+    __shared__ sdfo_body_state sA, sB;
+    __shared__ Place32 s_place;
+    __shared__ BroadShared s_broad;
+    __shared__ MeasureShared<T / 32> s_meas;
+    load_states(poses + pose, body_b, sA, sB);
+    __syncthreads();
+    const PoseFrame f = pose_frame(sA, sB);
+    Place32 at;
+    if (HOW != kEveryPoint)
+    {
+        set_place_entry(g, sA, sB, f.tl, (int)threadIdx.x, s_place);
+        __syncthreads();
+        at = s_place;
+        at.set_margin(s_place.e0);
+    }
+    const bool full = broad_phase<T>(cull, sA, f, s_broad);
+    Measured seen;
+    auto kept = [&](int i) {
+        if (full) return true;
+        const int l = __ldg(cull.pleaf + i);
+        return ((s_broad.mask[l >> 5] >> (l & 31)) & 1u) != 0;
+    };
+    auto sample_point = [&](int i, float x, float y, float z) {
+        const v3 Yv = mulT(sB.R, mul(sA.R, V(x, y, z))) + f.tl;
+        const double Y[3] = {Yv.x, Yv.y, Yv.z};
+        float gap;
+        v3 gl;
+        double Hl[6];
+        if (sample<MODE, SPARSE, BD, false>(g, Y, gap, gl, Hl)) seen.point(cull, full, i, gap);
+    };
+    float least = INFINITY; // no gap above it is needed
+    for (int i0 = 0; i0 < nq; i0 += T) // the same trips for every lane of a warp
+    {
+        const int i = i0 + (int)threadIdx.x;
+        const bool in = i < nq && kept(i);
+        float x = 0.f, y = 0.f, z = 0.f;
+        if (in)
+        {
+            x = __ldg(qx + 3 * i);
+            y = __ldg(qx + 3 * i + 1);
+            z = __ldg(qx + 3 * i + 2);
+        }
+        bool open = in;
+        if (HOW == kByBounds)
+        {
+            float gap = 0.f, eps = 0.f;
+            bool out = false;
+            const bool known = in && gap32(g, at, x, y, z, gap, eps, out);
+            least = warp_least(known ? fminf(least, gap + eps) : least);
+            const bool below = gap + eps < 0.f; // certainly active
+            if (known && gap - eps > least && (gap - eps > 0.f || below))
+            {
+                ++seen.nvalid;
+                if (below) ++seen.nactive;
+                open = false;
+            }
+            open = open && !out;
+        }
+        if (HOW == kByTouch)
+        {
+            const int status = touch_status(g, bits, at, x, y, z);
+            if (in && status == kClear) ++seen.nvalid;
+            open = in && status == kMayTouch;
+        }
+        if (open) sample_point(i, x, y, z);
+    }
+    if (HOW == kByTouch && __syncthreads_or(seen.best.gap <= 0.0) == 0)
+    {
+        // clear of the surface: the least gap may be among the points left out
+        seen = Measured{};
+        for (int i = threadIdx.x; i < nq; i += T)
+            if (kept(i)) sample_point(i, __ldg(qx + 3 * i), __ldg(qx + 3 * i + 1), __ldg(qx + 3 * i + 2));
+    }
+    write_measure<MODE, SPARSE, BD, T>(g, qx, sA, sB, f, cull, full, s_broad, s_meas, seen, meas + pose);
+}
+
 struct ContactLaunch
 {
     const float* qx;
@@ -932,9 +1041,44 @@ void launch3(const GridView& v, const ContactLaunch& c, const uint32_t* bits, cu
         launch4<MODE, SPARSE, BD, false, TOUCH>(v, c, bits, s);
 }
 
+// Resident CTAs per SM asked of the register allocator for a measure (256 threads
+// each): 4,096 clear poses, Trilinear 351 / 289 / 275 us at 3 / 4 / 5, Tricubic 539 /
+// 477 / 529.
+#ifndef SDFO_MEASURE_MIN_BLOCKS
+#define SDFO_MEASURE_MIN_BLOCKS 4
+#endif
+
+template <int MODE, bool SPARSE, int BD, int HOW>
+void launch_measure(const GridView& v, const ContactLaunch& c, const uint32_t* bits, cudaStream_t s)
+{
+    if (c.np <= current_sm_count())
+        k_measure<MODE, SPARSE, BD, HOW, kFewThreads, 1><<<c.np, kFewThreads, 0, s>>>(v, c.qx, c.nq, c.pa, c.pb, c.cull,
+                                                                                      c.meas, bits);
+    else
+        k_measure<MODE, SPARSE, BD, HOW, kContactThreads, SDFO_MEASURE_MIN_BLOCKS>
+            <<<c.np, kContactThreads, 0, s>>>(v, c.qx, c.nq, c.pa, c.pb, c.cull, c.meas, bits);
+}
+
 template <int MODE>
 void launch2(const GridView& v, const ContactLaunch& c, cudaStream_t s)
 {
+    if (c.meas && !c.ft)
+    {
+        // the touch bits and records of a grid that owns its payload
+        const int64_t voxels = (int64_t)v.nx * v.ny * v.nz;
+        const bool owned = v.layout == SDFO_LAYOUT_DENSE && v.touch && v.cell8 && voxels < (int64_t(1) << 31);
+        if (v.layout != SDFO_LAYOUT_DENSE && v.bd == 8)
+            launch_measure<MODE, true, 8, kEveryPoint>(v, c, nullptr, s);
+        else if (v.layout != SDFO_LAYOUT_DENSE)
+            launch_measure<MODE, true, 0, kEveryPoint>(v, c, nullptr, s);
+        else if (!owned)
+            launch_measure<MODE, false, 0, kEveryPoint>(v, c, nullptr, s);
+        else if constexpr (MODE == SDFO_TRICUBIC)
+            launch_measure<MODE, false, 0, kByTouch>(v, c, v.touch + touch_words(voxels), s);
+        else
+            launch_measure<MODE, false, 0, kByBounds>(v, c, nullptr, s);
+        return;
+    }
     if (v.layout == SDFO_LAYOUT_DENSE)
     {
         // The touch bits say where the gap can be <= 0; they leave out points
