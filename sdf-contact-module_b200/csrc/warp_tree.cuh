@@ -75,14 +75,25 @@ struct RayBins
     const int* off;    // CSR over the cells of all levels
     const int* ids;    // slots
     double e1[3], e2[3], o1, o2; // plane axes and lower corner
+    double o3;         // the scene's middle along the ray
     double size;       // side of the plane's square
     double inv_cell;   // finest cells per unit length
     int g;             // finest cells per side (a power of two)
 };
 
+// What FP32 sees of the scene: points relative to its middle `o`, so that an
+// offset from the origin costs no bits.  E: the half extent of mesh and grid
+// about `o`; far: their largest coordinate.  FP64 differences to `o` are rounded
+// to less than 2^-52 far.
+struct Scene32
+{
+    double o[3], e, far;
+};
+
 struct WarpTreeView
 {
     RefTreeView ref;
+    double o[3];         // Scene32::o
     const float4* node4; // 4 float4 per node: both child boxes, child codes
     const float4* tri4;  // 5 float4 per slot: the triangle in its own frame (k_tri_frames)
     float bound_abs;     // warp_bound's absolute part, rounded up
@@ -123,9 +134,13 @@ __global__ void k_mark_unbounded(RefTreeView b, int* __restrict__ flags, int* __
     }
 }
 
-// {L.lo, L.hi, R.lo, R.hi} in FP32, rounded outward and widened by the cull
-// margin, then the child codes: a node id, or ~id of a leaf.
-__global__ void k_pack_node4(RefTreeView b, const int* __restrict__ flags, float4* __restrict__ out)
+// Rounding of a point, a box or a distance that does not grow with the distance.
+inline double scene_margin(const Scene32& c) { return std::ldexp(c.e, -20) + std::ldexp(c.far, -50); }
+
+// {L.lo, L.hi, R.lo, R.hi} in FP32, rounded outward and widened by the margin,
+// then the child codes: a node id, or ~id of a leaf.
+__global__ void k_pack_node4(RefTreeView b, Scene32 sc, double margin, const int* __restrict__ flags,
+                             float4* __restrict__ out)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= b.nnodes) return;
@@ -139,8 +154,8 @@ __global__ void k_pack_node4(RefTreeView b, const int* __restrict__ flags, float
         const RefNode& c = b.nodes[ch[k]];
         for (int a = 0; a < 3; ++a)
         {
-            f[6 * k + a] = flags[ch[k]] ? -INFINITY : __double2float_rd(c.lo[a] - (double)b.cull_m);
-            f[6 * k + 3 + a] = flags[ch[k]] ? INFINITY : __double2float_ru(c.hi[a] + (double)b.cull_m);
+            f[6 * k + a] = flags[ch[k]] ? -INFINITY : __double2float_rd(c.lo[a] - sc.o[a] - margin);
+            f[6 * k + 3 + a] = flags[ch[k]] ? INFINITY : __double2float_ru(c.hi[a] - sc.o[a] + margin);
         }
         code[k] = c.count > 0 ? ~ch[k] : ch[k];
     }
@@ -156,7 +171,7 @@ __global__ void k_pack_node4(RefTreeView b, const int* __restrict__ flags, float
 // length of ab, unit directions and lengths of ac and bc in the plane, and the
 // part of TriPoint's error that does not depend on the point.
 // Near-degenerate triangles get a negative length of ab: never culled.
-__global__ void k_tri_frames(RefTreeView b, float frame_m, float4* __restrict__ out)
+__global__ void k_tri_frames(RefTreeView b, Scene32 sc, float frame_m, float4* __restrict__ out)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= b.n) return;
@@ -178,7 +193,7 @@ __global__ void k_tri_frames(RefTreeView b, float frame_m, float4* __restrict__ 
     const d3 z = unit(cross(sub(v[1], v[0]), ac), ln);
     const d3 y = cross(z, x);
     const d3 uac = unit(ac, lac), ubc = unit(bc, lbc);
-    o[0] = make_float4((float)v[0].x, (float)v[0].y, (float)v[0].z, (float)x.x);
+    o[0] = make_float4((float)(v[0].x - sc.o[0]), (float)(v[0].y - sc.o[1]), (float)(v[0].z - sc.o[2]), (float)x.x);
     o[1] = make_float4((float)x.y, (float)x.z, (float)y.x, (float)y.y);
     o[2] = make_float4((float)y.z, (float)z.x, (float)z.y, (float)z.z);
     o[3] = make_float4((float)lab, (float)dot(uac, x), (float)dot(uac, y), (float)lac);
@@ -305,10 +320,11 @@ __device__ __forceinline__ int level_base(int g, int level)
 // Triangle `s` on the plane.  Returns false when the reference's test can
 // never count it (|det| below its eps).  `grow` bounds how far outside the
 // triangle the FP64 test's rounding may still accept a point: with
-// u, v >= -eps - err / |det|, err < 2^-48 E |e|, the accepted points lie
-// within 3 (1e-12 + err / |det|) (|e1| + |e2|) of the triangle.
-__device__ bool project_triangle(const RefTreeView& b, const RayBins& r, double extent, int s, double q[6],
-                                 double depth[3], double& grow)
+// u, v >= -eps - err / |det|, err < 2^-48 E |e| (the test takes differences of
+// points, whose rounding is relative to them), the accepted points lie within
+// 3 (1e-12 + err / |det|) (|e1| + |e2|) of the triangle; `len` is the last factor.
+__device__ bool project_triangle(const RefTreeView& b, const RayBins& r, const Scene32& sc, int s, double q[6],
+                                 double depth[3], double& len, double& grow)
 {
     const d3 dir = mk(b.dir[0], b.dir[1], b.dir[2]);
     d3 v[3];
@@ -320,20 +336,20 @@ __device__ bool project_triangle(const RefTreeView& b, const RayBins& r, double 
     {
         q[2 * k] = dot(v[k], mk(r.e1[0], r.e1[1], r.e1[2])) - r.o1;
         q[2 * k + 1] = dot(v[k], mk(r.e2[0], r.e2[1], r.e2[2])) - r.o2;
-        depth[k] = dot(v[k], dir);
+        depth[k] = dot(v[k], dir) - r.o3;
     }
-    const double len = sqrt(dot(e1, e1)) + sqrt(dot(e2, e2));
-    grow = 3.0 * (1.0e-12 + 0x1p-48 * extent * len / fabs(det)) * len + 0x1p-20 * r.size + 0x1p-44 * extent;
+    len = sqrt(dot(e1, e1)) + sqrt(dot(e2, e2));
+    grow = 3.0 * (1.0e-12 + 0x1p-48 * sc.e * len / fabs(det)) * len + 0x1p-20 * r.size + 0x1p-44 * sc.far;
     return true;
 }
 
-__global__ void k_ray_count(RefTreeView b, RayBins r, double extent, float4* __restrict__ rec,
+__global__ void k_ray_count(RefTreeView b, RayBins r, Scene32 sc, float4* __restrict__ rec,
                             int* __restrict__ counts, int* __restrict__ state)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= b.n) return;
-    double q[6], depth[3], grow;
-    if (!project_triangle(b, r, extent, s, q, depth, grow)) return;
+    double q[6], depth[3], len, grow;
+    if (!project_triangle(b, r, sc, s, q, depth, len, grow)) return;
     // the plane has a margin of 2^-10 of its side about the mesh's box
     if (!(grow < 0x1p-11 * r.size))
     {
@@ -344,11 +360,11 @@ __global__ void k_ray_count(RefTreeView b, RayBins r, double extent, float4* __r
     const int level = cell_level(r, p);
     // edge functions in FP32: coordinates are rounded by at most 2^-25 size,
     // differences are bounded by L for every origin in the triangle's cells,
-    // and the rounding of the products sums to less than 40 2^-24 L size; tol
-    // also covers the reference's own tolerance
+    // and the rounding of the products sums to less than 40 2^-24 L size; the FP64
+    // test accepts edge functions down to -(1e-12 |det| + err)
     const double L = (p.x1 - p.x0) + (p.y1 - p.y0) + 2.0 * ldexp(1.0 / r.inv_cell, level);
-    const double tol = L * (r.size * 0x1p-17 + extent * 0x1p-44);
-    const double deep = fmax(depth[0], fmax(depth[1], depth[2])) + grow + 0x1p-18 * extent;
+    const double tol = L * (r.size * 0x1p-17 + sc.far * 0x1p-44) + 0x1p-46 * sc.e * len;
+    const double deep = fmax(depth[0], fmax(depth[1], depth[2])) + grow + 0x1p-18 * sc.e;
     rec[2 * (int64_t)s] = make_float4((float)p.x[0], (float)p.y[0], (float)p.x[1], (float)p.y[1]);
     rec[2 * (int64_t)s + 1] =
         make_float4((float)p.x[2], (float)p.y[2], __double2float_ru(deep), __double2float_ru(tol));
@@ -357,13 +373,13 @@ __global__ void k_ray_count(RefTreeView b, RayBins r, double extent, float4* __r
     for_cells(r, p, level, [&](int c) { atomicAdd(counts + base + c, 1); });
 }
 
-__global__ void k_ray_emit(RefTreeView b, RayBins r, double extent, int* __restrict__ cursor,
+__global__ void k_ray_emit(RefTreeView b, RayBins r, Scene32 sc, int* __restrict__ cursor,
                            int* __restrict__ ids)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= b.n) return;
-    double q[6], depth[3], grow;
-    if (!project_triangle(b, r, extent, s, q, depth, grow)) return;
+    double q[6], depth[3], len, grow;
+    if (!project_triangle(b, r, sc, s, q, depth, len, grow)) return;
     if (!(grow < 0x1p-11 * r.size)) return;
     const PlaneTri p(q, grow);
     const int level = cell_level(r, p), base = level_base(r.g, level);
@@ -382,7 +398,7 @@ __device__ __forceinline__ int binned_ray_count(const WarpTreeView& t, const d3&
     const double q1 = dot(p, mk(r.e1[0], r.e1[1], r.e1[2])) - r.o1;
     const double q2 = dot(p, mk(r.e2[0], r.e2[1], r.e2[2])) - r.o2;
     if (!(q1 >= 0.0 && q1 < r.size && q2 >= 0.0 && q2 < r.size)) return 0;
-    const float qx = (float)q1, qy = (float)q2, depth = (float)dot(p, dir);
+    const float qx = (float)q1, qy = (float)q2, depth = (float)(dot(p, dir) - r.o3);
     const int cx = min((int)(q1 * r.inv_cell), r.g - 1), cy = min((int)(q2 * r.inv_cell), r.g - 1);
     int hits = 0, base = 0, gl = r.g;
     for (int levels = t.state[kStateLevels], l = 0; levels != 0; levels >>= 1, ++l)
@@ -547,10 +563,10 @@ __device__ __forceinline__ float gap2(const float p[3], float lx, float ly, floa
 
 // Triangle s in FP32.  In the triangle's frame the squared distance is z^2
 // plus the planar one.  Errors, in units of 2^-24: p and a are rounded to E per
-// axis; their difference, the rotation, the segments of ab and ac and the root
-// add less than 17 r, r = |x| + |y| + |z|; the segment of bc, 8 |ab|.  So the
-// distance to the plane, to an edge's line or to a segment is known to within
-// m = 2^-20 (E + r + |ab|).
+// axis (and to 2^-52 far beforehand); their difference, the rotation, the
+// segments of ab and ac and the root add less than 17 r, r = |x| + |y| + |z|; the
+// segment of bc, 8 |ab|.  So the distance to the plane, to an edge's line or to a
+// segment is known to within m = 2^-20 (E + r + |ab|) + 2^-50 far.
 struct TriFrame
 {
     float4 q0, q1, q2, q3, q4;
@@ -911,9 +927,9 @@ __global__ void __launch_bounds__(kFillThreads, SDFO_WARP_FILL_MIN_BLOCKS)
         int64_t idx = -1;
         const bool active = patch + k < patches && job.voxel(patch + k, lane, c, idx);
         if (!active) job.outside(idx);
-        pf[k][0] = (float)c.x;
-        pf[k][1] = (float)c.y;
-        pf[k][2] = (float)c.z;
+        pf[k][0] = (float)(c.x - t.o[0]);
+        pf[k][1] = (float)(c.y - t.o[1]);
+        pf[k][2] = (float)(c.z - t.o[2]);
         bound[k] = active ? INFINITY : -1.f;
     }
     const bool done = warp_search<false>(t, t.ref.nnodes == 1 ? ~0 : 0, stacks[warp], tris[warp], pf, bound, n, list, low, status,
@@ -979,9 +995,9 @@ __global__ void __launch_bounds__(32 * kHeavyWarps, 3) k_heavy_fill(Job job, int
             d3 c = mk(0.0, 0.0, 0.0);
             int64_t idx = -1;
             const bool active = patch + k < patches && job.voxel(patch + k, lane, c, idx);
-            pf[k][0] = (float)c.x;
-            pf[k][1] = (float)c.y;
-            pf[k][2] = (float)c.z;
+            pf[k][0] = (float)(c.x - t.o[0]);
+            pf[k][1] = (float)(c.y - t.o[1]);
+            pf[k][2] = (float)(c.z - t.o[2]);
             bound[k] = active ? job.phin[idx].y : -1.f;
             s_sq[warp][32 * k + lane] = DBL_MAX;
             s_slot[warp][32 * k + lane] = kNoSlot;
@@ -1156,12 +1172,23 @@ struct DeviceWarpTree
     WarpTreeView v{};
 
     // `tree`: uploaded nodes, slot-order triangles and triangle boxes; lo, hi:
-    // the mesh's box.
-    void build(const RefTreeView& tree, const double lo[3], const double hi[3], double extent, cudaStream_t s)
+    // the mesh's box; far: the largest coordinate of mesh and grid.
+    void build(const RefTreeView& tree, const double lo[3], const double hi[3], const sdfo_grid_info& grid, double far,
+               cudaStream_t s)
     {
         const int n = tree.n, T = 256;
+        Scene32 sc{};
+        sc.far = far;
+        for (int a = 0; a < 3; ++a)
+        {
+            const double l = std::min(lo[a], grid.bmin[a]), h = std::max(hi[a], grid.bmax[a]);
+            v.o[a] = sc.o[a] = 0.5 * l + 0.5 * h;
+            sc.e = std::max(sc.e, 0.5 * h - 0.5 * l);
+        }
+        const double margin = scene_margin(sc);
         v.ref = tree;
         v.rays = ray_plane(tree.dir, lo, hi, n);
+        for (int a = 0; a < 3; ++a) v.rays.o3 += sc.o[a] * tree.dir[a];
         const int cells = ray_cells(v.rays.g);
         node4.reset(4 * (size_t)tree.nnodes);
         tri4.reset(5 * (size_t)n);
@@ -1177,22 +1204,25 @@ struct DeviceWarpTree
         SDFO_CUDA(cudaMemsetAsync(counts.get(), 0, sizeof(int) * ((size_t)cells + 1), s));
         k_mark_unbounded<<<(n + T - 1) / T, T, 0, s>>>(tree, flags.get(), state.get());
         SDFO_CHECK_LAUNCH();
-        k_pack_node4<<<(tree.nnodes + T - 1) / T, T, 0, s>>>(tree, flags.get(), node4.get());
+        k_pack_node4<<<(tree.nnodes + T - 1) / T, T, 0, s>>>(tree, sc, margin, flags.get(), node4.get());
         SDFO_CHECK_LAUNCH();
-        k_tri_frames<<<(n + T - 1) / T, T, 0, s>>>(tree, (float)std::ldexp(extent, -20), tri4.get());
+        k_tri_frames<<<(n + T - 1) / T, T, 0, s>>>(tree, sc, (float)(margin * (1.0 + 0x1p-20)), tri4.get());
         SDFO_CHECK_LAUNCH();
-        k_ray_count<<<(n + T - 1) / T, T, 0, s>>>(tree, v.rays, extent, rec.get(), counts.get(), state.get());
+        k_ray_count<<<(n + T - 1) / T, T, 0, s>>>(tree, v.rays, sc, rec.get(), counts.get(), state.get());
         SDFO_CHECK_LAUNCH();
         size_t temp = 0;
         SDFO_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, temp, counts.get(), off.get(), cells + 1, s));
         scan.reset(temp);
         SDFO_CUDA(cub::DeviceScan::ExclusiveSum(scan.get(), temp, counts.get(), off.get(), cells + 1, s));
         SDFO_CUDA(cudaMemcpyAsync(counts.get(), off.get(), sizeof(int) * (size_t)cells, cudaMemcpyDeviceToDevice, s));
-        k_ray_emit<<<(n + T - 1) / T, T, 0, s>>>(tree, v.rays, extent, counts.get(), ids.get());
+        k_ray_emit<<<(n + T - 1) / T, T, 0, s>>>(tree, v.rays, sc, counts.get(), ids.get());
         SDFO_CHECK_LAUNCH();
         v.node4 = node4.get();
         v.tri4 = tri4.get();
-        v.bound_abs = (float)(tree.cull_abs * (1.0 + 0x1p-15));
+        // what the FP64 closest point of a well-conditioned triangle can be off by
+        // beside 2^-16 of its squared distance: (2^-20 E)^2, and for coordinates
+        // far from the origin, whose rounding is 2^-52 far, (2^-40 far)^2
+        v.bound_abs = (float)((std::ldexp(sc.e * sc.e, -40) + std::ldexp(far * far, -80)) * (1.0 + 0x1p-15));
         v.rays.rec = rec.get();
         v.rays.off = off.get();
         v.rays.ids = ids.get();
