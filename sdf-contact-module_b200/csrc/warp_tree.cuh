@@ -97,41 +97,28 @@ struct WarpTreeView
     const float4* node4; // 4 float4 per node: both child boxes, child codes
     const float4* tri4;  // 5 float4 per slot: the triangle in its own frame (k_tri_frames)
     float bound_abs;     // warp_bound's absolute part, rounded up
+    const int* unbounded; // slots of the near-degenerate triangles
     int* heavy;          // first patches of the pairs handed over
     RayBins rays;
     int* state;
 };
 
+__device__ __forceinline__ bool too_many_unbounded(const int* state) { return state[kStateUnbounded] > kMaxUnbounded; }
+
 __device__ __forceinline__ bool warp_path_open(const WarpTreeView& t)
 {
-    return t.state[kStateUnbounded] <= kMaxUnbounded && t.state[kStateWild] == 0;
+    return !too_many_unbounded(t.state) && t.state[kStateWild] == 0;
 }
 
-// Near-degenerate triangles (k_tri_boxes gives them an unbounded box) counted,
-// and every node on the way to one flagged: its box must not cull either.
-__global__ void k_mark_unbounded(RefTreeView b, int* __restrict__ flags, int* __restrict__ state)
+// Near-degenerate triangles (k_tri_boxes gives them an unbounded box): their
+// computed distance may be anything, so FP32 bounds nothing.  They stay out of
+// the search, and every voxel takes the FP64 test of each.
+__global__ void k_list_unbounded(RefTreeView b, int* __restrict__ list, int* __restrict__ state)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= b.n || b.tbox[2 * (int64_t)s].x != -INFINITY) return;
-    if (atomicAdd(state + kStateUnbounded, 1) >= kMaxUnbounded) return;
-    int node = 0, lo = 0, hi = b.n;
-    for (;;)
-    {
-        flags[node] = 1;
-        const int4 meta = __ldg(reinterpret_cast<const int4*>(b.nodes + node) + 3);
-        if (meta.w > 0) return;
-        const int mid = lo + (hi - lo) / 2;
-        if (s < mid)
-        {
-            node = meta.x;
-            hi = mid;
-        }
-        else
-        {
-            node = meta.y;
-            lo = mid;
-        }
-    }
+    const int k = atomicAdd(state + kStateUnbounded, 1);
+    if (k < kMaxUnbounded) list[k] = s;
 }
 
 // Rounding of a point, a box or a distance that does not grow with the distance.
@@ -139,11 +126,11 @@ inline double scene_margin(const Scene32& c) { return std::ldexp(c.e, -20) + std
 
 // {L.lo, L.hi, R.lo, R.hi} in FP32, rounded outward and widened by the margin,
 // then the child codes: a node id, or ~id of a leaf.
-__global__ void k_pack_node4(RefTreeView b, Scene32 sc, double margin, const int* __restrict__ flags,
+__global__ void k_pack_node4(RefTreeView b, Scene32 sc, double margin, const int* __restrict__ state,
                              float4* __restrict__ out)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= b.nnodes) return;
+    if (i >= b.nnodes || too_many_unbounded(state)) return;
     const int4 meta = __ldg(reinterpret_cast<const int4*>(b.nodes + i) + 3);
     if (meta.w > 0) return;
     const int ch[2] = {meta.x, meta.y};
@@ -154,8 +141,8 @@ __global__ void k_pack_node4(RefTreeView b, Scene32 sc, double margin, const int
         const RefNode& c = b.nodes[ch[k]];
         for (int a = 0; a < 3; ++a)
         {
-            f[6 * k + a] = flags[ch[k]] ? -INFINITY : __double2float_rd(c.lo[a] - sc.o[a] - margin);
-            f[6 * k + 3 + a] = flags[ch[k]] ? INFINITY : __double2float_ru(c.hi[a] - sc.o[a] + margin);
+            f[6 * k + a] = __double2float_rd(c.lo[a] - sc.o[a] - margin);
+            f[6 * k + 3 + a] = __double2float_ru(c.hi[a] - sc.o[a] + margin);
         }
         code[k] = c.count > 0 ? ~ch[k] : ch[k];
     }
@@ -170,11 +157,12 @@ __global__ void k_pack_node4(RefTreeView b, Scene32 sc, double margin, const int
 // rotation to (along ab, in the plane across ab towards c, the normal), the
 // length of ab, unit directions and lengths of ac and bc in the plane, and the
 // part of TriPoint's error that does not depend on the point.
-// Near-degenerate triangles get a negative length of ab: never culled.
-__global__ void k_tri_frames(RefTreeView b, Scene32 sc, float frame_m, float4* __restrict__ out)
+// Near-degenerate triangles get a negative length of ab: left out.
+__global__ void k_tri_frames(RefTreeView b, Scene32 sc, float frame_m, const int* __restrict__ state,
+                             float4* __restrict__ out)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= b.n) return;
+    if (s >= b.n || too_many_unbounded(state)) return;
     const d3 v[3] = {tri_vertex(b, s, 0), tri_vertex(b, s, 1), tri_vertex(b, s, 2)};
     float4* o = out + 5 * (int64_t)s;
     if (b.tbox[2 * (int64_t)s].x == -INFINITY)
@@ -347,7 +335,7 @@ __global__ void k_ray_count(RefTreeView b, RayBins r, Scene32 sc, float4* __rest
                             int* __restrict__ counts, int* __restrict__ state)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= b.n) return;
+    if (s >= b.n || too_many_unbounded(state)) return;
     double q[6], depth[3], len, grow;
     if (!project_triangle(b, r, sc, s, q, depth, len, grow)) return;
     // the plane has a margin of 2^-10 of its side about the mesh's box
@@ -373,11 +361,11 @@ __global__ void k_ray_count(RefTreeView b, RayBins r, Scene32 sc, float4* __rest
     for_cells(r, p, level, [&](int c) { atomicAdd(counts + base + c, 1); });
 }
 
-__global__ void k_ray_emit(RefTreeView b, RayBins r, Scene32 sc, int* __restrict__ cursor,
-                           int* __restrict__ ids)
+__global__ void k_ray_emit(RefTreeView b, RayBins r, Scene32 sc, const int* __restrict__ state,
+                           int* __restrict__ cursor, int* __restrict__ ids)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= b.n) return;
+    if (s >= b.n || too_many_unbounded(state)) return;
     double q[6], depth[3], len, grow;
     if (!project_triangle(b, r, sc, s, q, depth, len, grow)) return;
     if (!(grow < 0x1p-11 * r.size)) return;
@@ -552,7 +540,23 @@ __device__ __forceinline__ void flush_list(const WarpTreeView& t, const d3& p, i
     r.slot = ties == 1 && r.slot < 0 ? list[0] : first_visited(t.ref, p, list, ties, r.slot);
 }
 
-// Lower bound of the squared distance to a box widened by the cull margin.
+// The near-degenerate triangles after all others; the list's space is used up.
+__device__ __forceinline__ void flush_unbounded(const WarpTreeView& t, const d3& p, int* list, float* low, LaneNearest& r)
+{
+    const int count = t.state[kStateUnbounded];
+    for (int base = 0; base < count; base += kLaneList)
+    {
+        const int n = min(kLaneList, count - base);
+        for (int k = 0; k < n; ++k)
+        {
+            list[32 * k] = __ldg(t.unbounded + base + k);
+            low[32 * k] = 0.f;
+        }
+        flush_list(t, p, list, low, n, 0.f, r);
+    }
+}
+
+// Lower bound of the squared distance to a box widened by the margin.
 __device__ __forceinline__ float gap2(const float p[3], float lx, float ly, float lz, float hx, float hy, float hz)
 {
     const float x = fmaxf(fmaxf(lx - p[0], p[0] - hx), 0.f);
@@ -571,7 +575,7 @@ struct TriFrame
 {
     float4 q0, q1, q2, q3, q4;
     __device__ __forceinline__ explicit TriFrame(const float4* q) : q0(q[0]), q1(q[1]), q2(q[2]), q3(q[3]), q4(q[4]) {}
-    __device__ __forceinline__ bool whole() const { return q3.x < 0.f; } // near-degenerate
+    __device__ __forceinline__ bool left_out() const { return q3.x < 0.f; } // near-degenerate
 };
 
 // One point against one triangle: first the cheap lower bound by the
@@ -594,7 +598,7 @@ struct TriPoint
     __device__ __forceinline__ bool need(const TriFrame& f, float bound) const
     {
         const float lz = fmaxf(fabsf(z) - m, 0.f), lo = fmaxf(side - m, 0.f);
-        return f.whole() || !(__fmaf_rn(lz, lz, lo * lo) > bound);
+        return !f.left_out() && !(__fmaf_rn(lz, lz, lo * lo) > bound);
     }
     // Bounds of the squared distance; false: the triangle cannot matter.
     // Otherwise `bound` is lowered to what this triangle attains: the distance
@@ -612,13 +616,10 @@ struct TriPoint
                                                                 __fmaf_rn(sbc, sbc, ebc * ebc)));
         const float d = sqrtf(__fmaf_rn(z, z, side > 0.f ? d2 : 0.f));
         low = fmaxf(d - m, 0.f);
-        low = f.whole() ? 0.f : low * low;
-        if (low > bound) return false;
-        if (!f.whole())
-        {
-            const float up = (side > 0.f || side < -m ? d : sqrtf(__fmaf_rn(z, z, d2))) + m;
-            bound = fminf(bound, __fmaf_ru(__fmul_ru(up, up), 1.f + 0x1p-15f, t.bound_abs));
-        }
+        low *= low;
+        if (f.left_out() || low > bound) return false;
+        const float up = (side > 0.f || side < -m ? d : sqrtf(__fmaf_rn(z, z, d2))) + m;
+        bound = fminf(bound, __fmaf_ru(__fmul_ru(up, up), 1.f + 0x1p-15f, t.bound_abs));
         return true;
     }
 };
@@ -949,6 +950,7 @@ __global__ void __launch_bounds__(kFillThreads, SDFO_WARP_FILL_MIN_BLOCKS)
         }
         LaneNearest w{DBL_MAX, -1, false};
         flush_list(t, c, list + k * kLaneList * 32, low + k * kLaneList * 32, k ? n[1] : n[0], bd, w);
+        flush_unbounded(t, c, list + k * kLaneList * 32, low + k * kLaneList * 32, w);
         bool ok = w.slot >= 0 && !w.unsure;
         const int hits = ok && !t.ref.pn ? binned_ray_count(t, c, &ok) : 0;
         if (!ok)
@@ -1060,6 +1062,7 @@ __global__ void __launch_bounds__(32 * kHeavyWarps, 3) k_heavy_fill(Job job, int
                     mine[32 * ties++] = kept < 0 ? ~kept : kept;
                 }
                 if (ties > 0) w.slot = ties == 1 ? mine[0] : first_visited(t.ref, c, mine, ties, -1);
+                flush_unbounded(t, c, mine, lows[v >> 5] + (v & 31), w);
                 bool ok = w.slot >= 0 && !w.unsure;
                 const int hits = ok && !t.ref.pn ? binned_ray_count(t, c, &ok) : 0;
                 if (ok)
@@ -1167,7 +1170,7 @@ inline int ray_cells(int g)
 struct DeviceWarpTree
 {
     DeviceBuffer<float4> node4, tri4, rec;
-    DeviceBuffer<int> off, ids, state, flags, counts, heavy;
+    DeviceBuffer<int> off, ids, state, unbounded, counts, heavy;
     DeviceBuffer<unsigned char> scan;
     WarpTreeView v{};
 
@@ -1197,16 +1200,16 @@ struct DeviceWarpTree
         ids.reset((size_t)n * kMaxCellsPerTri);
         state.reset(kStateWords);
         // kept until the build's end: a free waits for the device
-        flags.reset((size_t)tree.nnodes);
+        unbounded.reset(kMaxUnbounded);
         counts.reset((size_t)cells + 1);
         SDFO_CUDA(cudaMemsetAsync(state.get(), 0, sizeof(int) * kStateWords, s));
-        SDFO_CUDA(cudaMemsetAsync(flags.get(), 0, sizeof(int) * (size_t)tree.nnodes, s));
         SDFO_CUDA(cudaMemsetAsync(counts.get(), 0, sizeof(int) * ((size_t)cells + 1), s));
-        k_mark_unbounded<<<(n + T - 1) / T, T, 0, s>>>(tree, flags.get(), state.get());
+        k_list_unbounded<<<(n + T - 1) / T, T, 0, s>>>(tree, unbounded.get(), state.get());
         SDFO_CHECK_LAUNCH();
-        k_pack_node4<<<(tree.nnodes + T - 1) / T, T, 0, s>>>(tree, sc, margin, flags.get(), node4.get());
+        k_pack_node4<<<(tree.nnodes + T - 1) / T, T, 0, s>>>(tree, sc, margin, state.get(), node4.get());
         SDFO_CHECK_LAUNCH();
-        k_tri_frames<<<(n + T - 1) / T, T, 0, s>>>(tree, sc, (float)(margin * (1.0 + 0x1p-20)), tri4.get());
+        k_tri_frames<<<(n + T - 1) / T, T, 0, s>>>(tree, sc, (float)(margin * (1.0 + 0x1p-20)), state.get(),
+                                                    tri4.get());
         SDFO_CHECK_LAUNCH();
         k_ray_count<<<(n + T - 1) / T, T, 0, s>>>(tree, v.rays, sc, rec.get(), counts.get(), state.get());
         SDFO_CHECK_LAUNCH();
@@ -1215,7 +1218,7 @@ struct DeviceWarpTree
         scan.reset(temp);
         SDFO_CUDA(cub::DeviceScan::ExclusiveSum(scan.get(), temp, counts.get(), off.get(), cells + 1, s));
         SDFO_CUDA(cudaMemcpyAsync(counts.get(), off.get(), sizeof(int) * (size_t)cells, cudaMemcpyDeviceToDevice, s));
-        k_ray_emit<<<(n + T - 1) / T, T, 0, s>>>(tree, v.rays, sc, counts.get(), ids.get());
+        k_ray_emit<<<(n + T - 1) / T, T, 0, s>>>(tree, v.rays, sc, state.get(), counts.get(), ids.get());
         SDFO_CHECK_LAUNCH();
         v.node4 = node4.get();
         v.tri4 = tri4.get();
@@ -1227,6 +1230,7 @@ struct DeviceWarpTree
         v.rays.off = off.get();
         v.rays.ids = ids.get();
         v.state = state.get();
+        v.unbounded = unbounded.get();
     }
 
     template <class Job>
