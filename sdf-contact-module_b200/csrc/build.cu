@@ -25,6 +25,7 @@
 // The fills over the reference-order tree run warp-wide (warp_tree.cuh), with
 // the same results.
 #include <atomic>
+#include <climits>
 
 #include "warp_tree.cuh"
 
@@ -129,16 +130,19 @@ void get_fill_tile(int* lx, int* ly)
 
 namespace {
 // The warp-wide fill's data over `tree`, where the fills use it: the
-// reference-order tree with the triangle cull on (it needs the FP32 boxes),
-// from kWarpFillTris triangles.  Below that the per-thread traversal has
-// little to diverge over and its one launch is the cheaper: 12 triangles into
-// 64^3 voxels 0.056 ms against 0.065, 112 triangles 0.17 ms against 0.12
-// (fill alone, one B200).
-constexpr int kWarpFillTris = 64;
-bool build_warp_tree(DeviceWarpTree& w, const AnyTree& tree, const sdfo_grid_info& grid, cudaStream_t s)
+// reference-order tree with the triangle cull on (it needs the FP32 boxes), from
+// kWarpFillTris triangles and, where the number of voxels is known, a quarter as
+// many pairs of patches (64 voxels) as SMs.  Below that the per-thread traversal
+// has little to diverge over and its one launch is the cheaper.  Whole builds by
+// it and warp-wide: 128 triangles into 64 x 64 x 32 voxels 0.24 and 0.28 ms, 256
+// triangles 0.33 and 0.30; 3,072 triangles into 8 x 8 x 24 0.63 and 0.78, 4,608
+// into 24 x 24 x 8 1.31 and 0.80.
+constexpr int kWarpFillTris = 256;
+bool build_warp_tree(DeviceWarpTree& w, const AnyTree& tree, const sdfo_grid_info& grid, int64_t voxels, cudaStream_t s)
 {
     if (tree.mode == SDFO_BVH_LBVH || !triangle_cull() || tree.ref.n < kWarpFillTris ||
-        !std::isfinite(tree.ref.extent))
+        tree.ref.n > INT_MAX / kMaxCellsPerTri || !std::isfinite(tree.ref.extent) ||
+        voxels < 16 * (int64_t)current_sm_count())
         return false;
     w.build(tree.ref.view(), tree.ref.lo, tree.ref.hi, grid, tree.ref.extent, s);
     return true;
@@ -170,7 +174,7 @@ sdfo_grid* build_dense(const double* verts, int64_t nv, const int32_t* tris, int
     AnyTree tree{bvh_mode()};
     tree.build(verts, nv, tris, nt, scene_extent(verts, nv, g->info), s);
     DeviceWarpTree warp;
-    const bool warp_fill = build_warp_tree(warp, tree, g->info, s);
+    const bool warp_fill = build_warp_tree(warp, tree, g->info, N, s);
     g->stats.bvh_nodes = tree.node_count(nt);
     g->stats.bvh_ms = tm.lap();
     const SpecD sp = spec_of(g->info);
@@ -261,7 +265,7 @@ sdfo_grid* build_sparse(const double* verts, int64_t nv, const int32_t* tris, in
     AnyTree tree{bvh_mode()};
     tree.build(verts, nv, tris, nt, scene_extent(verts, nv, g->info), s);
     DeviceWarpTree warp;
-    const bool warp_fill = build_warp_tree(warp, tree, g->info, s);
+    const bool warp_fill = build_warp_tree(warp, tree, g->info, INT64_MAX, s);
     g->stats.bvh_nodes = tree.node_count(nt);
     g->stats.bvh_ms = tm.lap();
     DeviceBuffer<int> status(1);

@@ -19,7 +19,10 @@
 // A patch about equally far from much of the mesh (the axis of a cylinder)
 // enters hundreds of leaves, and one warp doing so outlasts the whole launch.
 // Such a patch stops after kHeavyLeaves leaves; in a second launch a CTA takes
-// it, its warps sharing out the subtrees.
+// it, its warps sharing out the subtrees.  Where there are no more pairs of
+// patches than such CTAs, every search is latency, and kFewLeaves hands over
+// sooner: 24 voxels along the longest side, 4,608 triangles of a cylinder 1.02 ->
+// 0.76 ms for the build, 9,016 of a gear 1.37 -> 1.02, 20,480 of a ball 2.3 -> 2.0.
 //
 // The parity ray has one fixed direction.  The triangles are projected along
 // it and binned on the plane; a voxel tests the triangles of its bin with FP32
@@ -29,15 +32,23 @@
 // Voxels for which the argument of flush_list or of binned_ray_count does
 // not hold (rounding at a box face) are marked and filled by the per-thread
 // traversal in a third launch, as are whole meshes with more than
-// kMaxUnbounded near-degenerate triangles.
+// kMaxUnbounded near-degenerate triangles, or whose long thin triangles crowd the
+// ray's lists (kMaxCrowd): a 1,024-triangle pipe ten diameters long has 421
+// entries where cylinders, gears and plates have 5 to 26, and its 64 x 64 x 128
+// voxels took 0.73 ms here, 0.54 per thread.
 //
 // Measured (one B200, fill alone): 34,816-triangle hollow cylinder into
 // 128 x 128 x 64 voxels 8.4 -> 2.0 ms; 327,680-triangle icosphere, 10.6 M
-// voxels of a sparse 512^3 grid, 37.9 -> 8.1 ms.  Bound now by instruction
+// voxels of a sparse 512^3 grid, 37.9 -> 8.1 ms.  Flat-faced parts gain nothing or
+// lose a little, since a point near a plane has few candidates (builds of cubes,
+// plates, rods and flat sheets of 768 to 12,288 triangles: 0.76 to 1.12 times the
+// per-thread speed, the least for the smallest grids).  Bound now by instruction
 // issue: 2.8 of 4 per cycle, about 34,000 per 64 voxels, of which a third FP32
 // and a tenth FP64 (81,920 triangles, 256^3).  A triangle-box test ahead of the
 // frame test changed nothing (7.2 against 7.3 ms).
 #pragma once
+
+#include <climits>
 
 #include "build_common.cuh"
 
@@ -49,14 +60,17 @@ constexpr int kMaxUnbounded = 32;
 constexpr int kWarpStack = 64;
 constexpr int kLeafTris = 8;      // triangles of a leaf of the reference's tree, at most
 constexpr int kLaneList = 8;      // triangles a lane keeps for the FP64 test
-constexpr int kHeavyLeaves = 128; // leaves after which a patch is handed over
+constexpr int kHeavyLeaves = 128; // leaves after which a patch is handed over,
+constexpr int kFewLeaves = 16;    // where all patches fit the CTAs at once
 constexpr int kHeavyWarps = 8;    // warps of the CTA that takes such a patch
+constexpr int kHeavyBlocks = 3;   // such CTAs per SM
 static_assert(kHeavyWarps <= kLaneList, "the warps' results are compared in a list");
 constexpr int kPartDepth = 6;     // depth of the subtrees they share out
 // Rays: a triangle goes to the finest level where it reaches at most this
 // many cells, so the lists hold at most this many entries per triangle.
 constexpr int kMaxCellsPerTri = 16;
 constexpr int kMaxRayCells = 1024; // cells per side of the finest level
+constexpr double kMaxCrowd = 128.0; // mean entries over the mesh's projected box
 
 // state words of a WarpTree
 enum : int
@@ -66,7 +80,8 @@ enum : int
     kStateLevels = 2,    // bit l: level l holds triangles
     kStateMarked = 3,    // voxels left to the per-thread traversal
     kStateHeavy = 4,     // pairs of patches handed over
-    kStateWords = 5
+    kStateCrowd = 6,     // (64 bits) area of all list entries' cells, in finest cells
+    kStateWords = 8
 };
 
 struct RayBins
@@ -76,6 +91,7 @@ struct RayBins
     const int* ids;    // slots
     double e1[3], e2[3], o1, o2; // plane axes and lower corner
     double o3;         // the scene's middle along the ray
+    double box_cells;  // area of the mesh's projected box, in finest cells
     double size;       // side of the plane's square
     double inv_cell;   // finest cells per unit length
     int g;             // finest cells per side (a power of two)
@@ -98,27 +114,17 @@ struct WarpTreeView
     const float4* tri4;  // 5 float4 per slot: the triangle in its own frame (k_tri_frames)
     float bound_abs;     // warp_bound's absolute part, rounded up
     const int* unbounded; // slots of the near-degenerate triangles
+    unsigned long long max_crowd; // of kStateCrowd
     int* heavy;          // first patches of the pairs handed over
+    int max_leaves;      // leaves after which a pair is
     RayBins rays;
     int* state;
 };
 
-__device__ __forceinline__ bool too_many_unbounded(const int* state) { return state[kStateUnbounded] > kMaxUnbounded; }
-
 __device__ __forceinline__ bool warp_path_open(const WarpTreeView& t)
 {
-    return !too_many_unbounded(t.state) && t.state[kStateWild] == 0;
-}
-
-// Near-degenerate triangles (k_tri_boxes gives them an unbounded box): their
-// computed distance may be anything, so FP32 bounds nothing.  They stay out of
-// the search, and every voxel takes the FP64 test of each.
-__global__ void k_list_unbounded(RefTreeView b, int* __restrict__ list, int* __restrict__ state)
-{
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= b.n || b.tbox[2 * (int64_t)s].x != -INFINITY) return;
-    const int k = atomicAdd(state + kStateUnbounded, 1);
-    if (k < kMaxUnbounded) list[k] = s;
+    return t.state[kStateUnbounded] <= kMaxUnbounded && t.state[kStateWild] == 0 &&
+           *reinterpret_cast<const unsigned long long*>(t.state + kStateCrowd) <= t.max_crowd;
 }
 
 // Rounding of a point, a box or a distance that does not grow with the distance.
@@ -126,11 +132,10 @@ inline double scene_margin(const Scene32& c) { return std::ldexp(c.e, -20) + std
 
 // {L.lo, L.hi, R.lo, R.hi} in FP32, rounded outward and widened by the margin,
 // then the child codes: a node id, or ~id of a leaf.
-__global__ void k_pack_node4(RefTreeView b, Scene32 sc, double margin, const int* __restrict__ state,
-                             float4* __restrict__ out)
+__global__ void k_pack_node4(RefTreeView b, Scene32 sc, double margin, float4* __restrict__ out)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= b.nnodes || too_many_unbounded(state)) return;
+    if (i >= b.nnodes) return;
     const int4 meta = __ldg(reinterpret_cast<const int4*>(b.nodes + i) + 3);
     if (meta.w > 0) return;
     const int ch[2] = {meta.x, meta.y};
@@ -158,11 +163,9 @@ __global__ void k_pack_node4(RefTreeView b, Scene32 sc, double margin, const int
 // length of ab, unit directions and lengths of ac and bc in the plane, and the
 // part of TriPoint's error that does not depend on the point.
 // Near-degenerate triangles get a negative length of ab: left out.
-__global__ void k_tri_frames(RefTreeView b, Scene32 sc, float frame_m, const int* __restrict__ state,
-                             float4* __restrict__ out)
+__device__ __forceinline__ void tri_frame(const RefTreeView& b, const Scene32& sc, float frame_m, int s,
+                                          float4* __restrict__ out)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= b.n || too_many_unbounded(state)) return;
     const d3 v[3] = {tri_vertex(b, s, 0), tri_vertex(b, s, 1), tri_vertex(b, s, 2)};
     float4* o = out + 5 * (int64_t)s;
     if (b.tbox[2 * (int64_t)s].x == -INFINITY)
@@ -192,11 +195,11 @@ __global__ void k_tri_frames(RefTreeView b, Scene32 sc, float frame_m, const int
 // ---------------------------------------------------------------------------
 // ray bins
 // ---------------------------------------------------------------------------
-// The triangle on the plane, counter-clockwise: corners and its box grown by
-// `grow`.
+// The triangle on the plane, counter-clockwise: corners, reciprocal heights of
+// its edges (0: flatter than `grow`) and its box grown by `grow`.
 struct PlaneTri
 {
-    double x[3], y[3], x0, x1, y0, y1, grow;
+    double x[3], y[3], inv[3], x0, x1, y0, y1, grow;
     __device__ PlaneTri(const double q[6], double g) : grow(g)
     {
         const bool turn = (q[2] - q[0]) * (q[5] - q[1]) - (q[3] - q[1]) * (q[4] - q[0]) < 0.0;
@@ -210,9 +213,16 @@ struct PlaneTri
         x1 = fmax(x[0], fmax(x[1], x[2])) + g;
         y0 = fmin(y[0], fmin(y[1], y[2])) - g;
         y1 = fmax(y[0], fmax(y[1], y[2])) + g;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+        {
+            const double d = y[k == 2 ? 0 : k + 1] - y[k];
+            inv[k] = fabs(d) > g ? 1.0 / d : 0.0;
+        }
     }
     // The x range of the grown triangle between the heights lo and hi: its
-    // edges clipped to the strip grown by `grow`, grown in x.
+    // edges clipped to the strip grown by `grow`, grown in x (by far more than
+    // the products are rounded).
     __device__ void strip(double lo, double hi, double& xl, double& xh) const
     {
         xl = DBL_MAX;
@@ -221,13 +231,13 @@ struct PlaneTri
         for (int k = 0; k < 3; ++k)
         {
             const int e = k == 2 ? 0 : k + 1;
-            const double a = y[k], d = y[e] - a;
+            const double a = y[k];
             if (fmax(a, y[e]) < lo - grow || fmin(a, y[e]) > hi + grow) continue;
             double t0 = 0.0, t1 = 1.0;
-            if (fabs(d) > grow)
+            if (inv[k] != 0.0)
             {
-                t0 = fmin(fmax((lo - grow - a) / d, 0.0), 1.0);
-                t1 = fmin(fmax((hi + grow - a) / d, 0.0), 1.0);
+                t0 = fmin(fmax((lo - grow - a) * inv[k], 0.0), 1.0);
+                t1 = fmin(fmax((hi + grow - a) * inv[k], 0.0), 1.0);
             }
             const double u = x[k] + t0 * (x[e] - x[k]), v = x[k] + t1 * (x[e] - x[k]);
             xl = fmin(xl, fmin(u, v));
@@ -261,7 +271,7 @@ __device__ __forceinline__ int for_cells(const RayBins& r, const PlaneTri& p, in
 {
     const CellBox b(r, p, level);
     const bool all = b.count() <= kMaxCellsPerTri;
-    const double w = ldexp(1.0 / r.inv_cell, level);
+    const double w = ldexp(1.0 / r.inv_cell, level), inv_w = ldexp(r.inv_cell, -level);
     int n = 0;
     for (int iy = b.y0; iy <= b.y1; ++iy)
     {
@@ -271,8 +281,8 @@ __device__ __forceinline__ int for_cells(const RayBins& r, const PlaneTri& p, in
             double xl, xh;
             p.strip(iy * w, (iy + 1) * w, xl, xh);
             if (!(xl <= xh)) continue;
-            x0 = max(x0, (int)fmax(floor(xl / w), 0.0));
-            x1 = min(x1, (int)fmax(floor(xh / w), 0.0));
+            x0 = max(x0, (int)fmax(floor(xl * inv_w), 0.0));
+            x1 = min(x1, (int)fmax(floor(xh * inv_w), 0.0));
         }
         for (int ix = x0; ix <= x1; ++ix)
         {
@@ -331,11 +341,24 @@ __device__ bool project_triangle(const RefTreeView& b, const RayBins& r, const S
     return true;
 }
 
-__global__ void k_ray_count(RefTreeView b, RayBins r, Scene32 sc, float4* __restrict__ rec,
-                            int* __restrict__ counts, int* __restrict__ state)
+// What there is per triangle (one thread each): its frame, its place in the list
+// if it is near-degenerate (k_tri_boxes gives it an unbounded box: its computed
+// distance may be anything, so FP32 bounds nothing; it stays out of the search,
+// and every voxel takes the FP64 test of each), and for the rays its record, its
+// level (-1: none) and the counts of its cells.
+__global__ void k_tri_tables(RefTreeView b, RayBins r, Scene32 sc, float frame_m, float4* __restrict__ tri4,
+                             int* __restrict__ unbounded, float4* __restrict__ rec, signed char* __restrict__ levels,
+                             int* __restrict__ counts, int* __restrict__ state)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= b.n || too_many_unbounded(state)) return;
+    if (s >= b.n) return;
+    tri_frame(b, sc, frame_m, s, tri4);
+    if (b.tbox[2 * (int64_t)s].x == -INFINITY)
+    {
+        const int k = atomicAdd(state + kStateUnbounded, 1);
+        if (k < kMaxUnbounded) unbounded[k] = s;
+    }
+    levels[s] = -1;
     double q[6], depth[3], len, grow;
     if (!project_triangle(b, r, sc, s, q, depth, len, grow)) return;
     // the plane has a margin of 2^-10 of its side about the mesh's box
@@ -356,22 +379,27 @@ __global__ void k_ray_count(RefTreeView b, RayBins r, Scene32 sc, float4* __rest
     rec[2 * (int64_t)s] = make_float4((float)p.x[0], (float)p.y[0], (float)p.x[1], (float)p.y[1]);
     rec[2 * (int64_t)s + 1] =
         make_float4((float)p.x[2], (float)p.y[2], __double2float_ru(deep), __double2float_ru(tol));
+    levels[s] = (signed char)level;
     atomicOr(state + kStateLevels, 1 << level);
     const int base = level_base(r.g, level);
-    for_cells(r, p, level, [&](int c) { atomicAdd(counts + base + c, 1); });
+    const int reached = for_cells(r, p, level, [&](int c) { atomicAdd(counts + base + c, 1); });
+    const unsigned lanes = __activemask();
+    const unsigned area = __reduce_add_sync(lanes, (unsigned)reached << (2 * level));
+    if ((int)(threadIdx.x & 31) == __ffs(lanes) - 1)
+        atomicAdd(reinterpret_cast<unsigned long long*>(state + kStateCrowd), (unsigned long long)area);
 }
 
-__global__ void k_ray_emit(RefTreeView b, RayBins r, Scene32 sc, const int* __restrict__ state,
-                           int* __restrict__ cursor, int* __restrict__ ids)
+// The lists' entries; counts go back to 0.
+__global__ void k_ray_emit(RefTreeView b, RayBins r, Scene32 sc, const signed char* __restrict__ levels,
+                           const int* __restrict__ off, int* __restrict__ counts, int* __restrict__ ids)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= b.n || too_many_unbounded(state)) return;
+    if (s >= b.n || levels[s] < 0) return;
     double q[6], depth[3], len, grow;
-    if (!project_triangle(b, r, sc, s, q, depth, len, grow)) return;
-    if (!(grow < 0x1p-11 * r.size)) return;
-    const PlaneTri p(q, grow);
-    const int level = cell_level(r, p), base = level_base(r.g, level);
-    for_cells(r, p, level, [&](int c) { ids[atomicAdd(cursor + base + c, 1)] = s; });
+    project_triangle(b, r, sc, s, q, depth, len, grow);
+    const int level = levels[s], base = level_base(r.g, level);
+    for_cells(r, PlaneTri(q, grow), level,
+              [&](int c) { ids[off[base + c] + atomicAdd(counts + base + c, -1) - 1] = s; });
 }
 
 // countRayIntersections by bins.  The reference tests a triangle when the
@@ -694,7 +722,7 @@ __device__ __forceinline__ bool warp_search(const WarpTreeView& t, int node, int
         }
         else
         {
-            if (!PART && (leaves == kHeavyLeaves || __any_sync(0xffffffffu, full))) return false;
+            if (!PART && (leaves == t.max_leaves || __any_sync(0xffffffffu, full))) return false;
             ++leaves;
             const int4 meta = __ldg(reinterpret_cast<const int4*>(b.nodes + ~node) + 3);
             // the leaf's records (at most 8) in one go: one latency instead of
@@ -969,7 +997,7 @@ __global__ void __launch_bounds__(kFillThreads, SDFO_WARP_FILL_MIN_BLOCKS)
 // the tree for all 64 voxels, as they become free, and keeps its own nearest
 // triangles; the warps' results are then compared.
 template <class Job>
-__global__ void __launch_bounds__(32 * kHeavyWarps, 3) k_heavy_fill(Job job, int64_t patches, int* status)
+__global__ void __launch_bounds__(32 * kHeavyWarps, kHeavyBlocks) k_heavy_fill(Job job, int64_t patches, int* status)
 {
     __shared__ float4 tris[kHeavyWarps][5 * kLeafTris];
     __shared__ int stacks[kHeavyWarps][kWarpStack];
@@ -1111,7 +1139,7 @@ void launch_warp_fill(const Job& job, int* status, cudaStream_t s)
     k_warp_fill<<<(unsigned)((patches + 2 * (kFillThreads / 32) - 1) / (2 * (kFillThreads / 32))), kFillThreads, 0, s>>>(
         job, patches, status);
     SDFO_CHECK_LAUNCH();
-    k_heavy_fill<<<(unsigned)current_sm_count() * 3, 32 * kHeavyWarps, 0, s>>>(job, patches, status);
+    k_heavy_fill<<<(unsigned)current_sm_count() * kHeavyBlocks, 32 * kHeavyWarps, 0, s>>>(job, patches, status);
     SDFO_CHECK_LAUNCH();
     k_rest_fill<<<blocks, 256, 0, s>>>(job, patches, status);
     SDFO_CHECK_LAUNCH();
@@ -1156,6 +1184,7 @@ inline RayBins ray_plane(const double dir[3], const double lo[3], const double h
     r.g = 1;
     while (r.g < kMaxRayCells && (int64_t)r.g * r.g < n) r.g *= 2;
     r.inv_cell = (double)r.g / r.size;
+    r.box_cells = 4.0 * half[0] * half[1] * r.inv_cell * r.inv_cell;
     return r;
 }
 
@@ -1169,9 +1198,8 @@ inline int ray_cells(int g)
 // The fast path's data of one reference-order tree.
 struct DeviceWarpTree
 {
-    DeviceBuffer<float4> node4, tri4, rec;
-    DeviceBuffer<int> off, ids, state, unbounded, counts, heavy;
-    DeviceBuffer<unsigned char> scan;
+    DeviceBuffer<unsigned char> mem; // one block: every free waits for the device
+    DeviceBuffer<int> heavy;
     WarpTreeView v{};
 
     // `tree`: uploaded nodes, slot-order triangles and triangle boxes; lo, hi:
@@ -1193,50 +1221,53 @@ struct DeviceWarpTree
         v.rays = ray_plane(tree.dir, lo, hi, n);
         for (int a = 0; a < 3; ++a) v.rays.o3 += sc.o[a] * tree.dir[a];
         const int cells = ray_cells(v.rays.g);
-        node4.reset(4 * (size_t)tree.nnodes);
-        tri4.reset(5 * (size_t)n);
-        rec.reset(2 * (size_t)n);
-        off.reset((size_t)cells + 1);
-        ids.reset((size_t)n * kMaxCellsPerTri);
-        state.reset(kStateWords);
-        // kept until the build's end: a free waits for the device
-        unbounded.reset(kMaxUnbounded);
-        counts.reset((size_t)cells + 1);
-        SDFO_CUDA(cudaMemsetAsync(state.get(), 0, sizeof(int) * kStateWords, s));
-        SDFO_CUDA(cudaMemsetAsync(counts.get(), 0, sizeof(int) * ((size_t)cells + 1), s));
-        k_list_unbounded<<<(n + T - 1) / T, T, 0, s>>>(tree, unbounded.get(), state.get());
-        SDFO_CHECK_LAUNCH();
-        k_pack_node4<<<(tree.nnodes + T - 1) / T, T, 0, s>>>(tree, sc, margin, state.get(), node4.get());
-        SDFO_CHECK_LAUNCH();
-        k_tri_frames<<<(n + T - 1) / T, T, 0, s>>>(tree, sc, (float)(margin * (1.0 + 0x1p-20)), state.get(),
-                                                    tri4.get());
-        SDFO_CHECK_LAUNCH();
-        k_ray_count<<<(n + T - 1) / T, T, 0, s>>>(tree, v.rays, sc, rec.get(), counts.get(), state.get());
-        SDFO_CHECK_LAUNCH();
         size_t temp = 0;
-        SDFO_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, temp, counts.get(), off.get(), cells + 1, s));
-        scan.reset(temp);
-        SDFO_CUDA(cub::DeviceScan::ExclusiveSum(scan.get(), temp, counts.get(), off.get(), cells + 1, s));
-        SDFO_CUDA(cudaMemcpyAsync(counts.get(), off.get(), sizeof(int) * (size_t)cells, cudaMemcpyDeviceToDevice, s));
-        k_ray_emit<<<(n + T - 1) / T, T, 0, s>>>(tree, v.rays, sc, state.get(), counts.get(), ids.get());
+        SDFO_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, temp, (int*)nullptr, (int*)nullptr, cells + 1, s));
+        size_t bytes = 0;
+        auto part = [&](size_t b) {
+            const size_t at = bytes;
+            bytes += (b + 255) / 256 * 256;
+            return at;
+        };
+        const size_t p_node4 = part(64 * (size_t)tree.nnodes), p_tri4 = part(80 * (size_t)n), p_rec = part(32 * (size_t)n),
+                     p_ids = part(4 * (size_t)n * kMaxCellsPerTri), p_off = part(4 * ((size_t)cells + 1)),
+                     p_levels = part((size_t)n), p_unbounded = part(4 * (size_t)kMaxUnbounded), p_scan = part(temp),
+                     p_state = part(4 * (size_t)kStateWords), p_counts = part(4 * ((size_t)cells + 1));
+        mem.reset(bytes);
+        unsigned char* m = mem.get();
+        float4 *node4 = (float4*)(m + p_node4), *tri4 = (float4*)(m + p_tri4), *rec = (float4*)(m + p_rec);
+        int *ids = (int*)(m + p_ids), *off = (int*)(m + p_off), *unbounded = (int*)(m + p_unbounded),
+            *state = (int*)(m + p_state), *counts = (int*)(m + p_counts);
+        signed char* levels = (signed char*)(m + p_levels);
+        SDFO_CUDA(cudaMemsetAsync(state, 0, bytes - p_state, s)); // state and counts
+        k_tri_tables<<<(n + T - 1) / T, T, 0, s>>>(tree, v.rays, sc, (float)(margin * (1.0 + 0x1p-20)), tri4, unbounded,
+                                                   rec, levels, counts, state);
         SDFO_CHECK_LAUNCH();
-        v.node4 = node4.get();
-        v.tri4 = tri4.get();
+        k_pack_node4<<<(tree.nnodes + T - 1) / T, T, 0, s>>>(tree, sc, margin, node4);
+        SDFO_CHECK_LAUNCH();
+        SDFO_CUDA(cub::DeviceScan::ExclusiveSum(m + p_scan, temp, counts, off, cells + 1, s));
+        k_ray_emit<<<(n + T - 1) / T, T, 0, s>>>(tree, v.rays, sc, levels, off, counts, ids);
+        SDFO_CHECK_LAUNCH();
+        v.node4 = node4;
+        v.tri4 = tri4;
         // what the FP64 closest point of a well-conditioned triangle can be off by
         // beside 2^-16 of its squared distance: (2^-20 E)^2, and for coordinates
         // far from the origin, whose rounding is 2^-52 far, (2^-40 far)^2
         v.bound_abs = (float)((std::ldexp(sc.e * sc.e, -40) + std::ldexp(far * far, -80)) * (1.0 + 0x1p-15));
-        v.rays.rec = rec.get();
-        v.rays.off = off.get();
-        v.rays.ids = ids.get();
-        v.state = state.get();
-        v.unbounded = unbounded.get();
+        v.rays.rec = rec;
+        v.rays.off = off;
+        v.rays.ids = ids;
+        v.state = state;
+        v.unbounded = unbounded;
+        v.max_crowd = tree.pn ? ULLONG_MAX : (unsigned long long)std::min(kMaxCrowd * v.rays.box_cells, 1e18);
     }
 
     template <class Job>
     void fill(Job job, int* status, cudaStream_t s)
     {
-        heavy.reset((size_t)(job.patches() + 1) / 2);
+        const int64_t pairs = (job.patches() + 1) / 2;
+        heavy.reset((size_t)pairs);
+        v.max_leaves = pairs <= kHeavyBlocks * (int64_t)current_sm_count() ? kFewLeaves : kHeavyLeaves;
         v.heavy = heavy.get();
         job.t = v;
         launch_warp_fill(job, status, s);
