@@ -32,9 +32,9 @@
 // interpolated gap can be <= 0 there (GridView::touch); a first pass places
 // every point in FP32 and lists those whose cell has the bit, or whose cell
 // FP32 cannot tell (place32.cuh), and only the listed points take the FP64
-// transform, the gather and the law, shared out over all warps.  4096 poses of
+// transform, the gather and the law, shared out over eight warps.  4096 poses of
 // a 7,680-point ring about a block's face, a quarter of them in contact: forces
-// and Jacobian 750 -> 281 us (one B200); bound by the latency of the few FP64
+// and Jacobian 767 -> 308 us (one B200); bound by the latency of the few FP64
 // steps of a pose, no longer by the 31 M gathers.
 #include <climits>
 
@@ -45,22 +45,26 @@ namespace sdfo {
 namespace {
 
 // Threads per pose: kContactThreads, or kFewThreads when every pose has an SM to
-// itself (fewer poses than SMs, touch bits): 33 poses of 7,680 points, forces
-// and then the measure, 78 us with 256 threads, 49 with 512 (4,096 poses with the
-// Jacobian: 299 us against 388).
+// itself (no more poses than SMs; forces with touch bits, every measure): 33 poses
+// of 7,680 points, forces and then the measure, 64 us with 256 threads, 53 with
+// 512, of which 50 are the host's.
 constexpr int kContactThreads = 256;
 constexpr int kFewThreads = 512;
 // Points are listed by spans of kJacSpan; then all warps share the span's list.
 constexpr int kJacSpan = 4096;
-// With touch bits, 32 consecutive points go to list (their number) mod kRows, 32
-// consecutive entries of the span's list to partial sum (their number) mod
-// kRows: a pose's sums run in one order whatever the threads per pose, so its
-// forces do not depend on the other poses of the call.
-constexpr int kRows = kFewThreads / 32;
+// A pose's sums run in one order whatever the threads per pose, so that its forces
+// do not depend on the other poses of the call.  Of a span's chunks of 32 points,
+// number c belongs to list c mod 8, in order; with 512 threads warps w and w + 8
+// list the first and the second half of list w.  Group k of 32 entries goes to
+// force sum k mod kForceRows, one warp's registers, and column or group k of the
+// Jacobian to sum k mod kJacRows.
+constexpr int kForceRows = kContactThreads / 32;
+constexpr int kJacRows = kFewThreads / 32;
 // Groups of 32 points in contact up to which the Jacobian's columns are shared out
 // over the warps, every column evaluating its points anew.  4,096 poses in light
-// contact (about four groups): 613 us with the columns shared out up to here, 766
-// up to eight groups; in deep contact shared-out columns took 6.1 ms against 5.0.
+// contact (about four groups): 0.58 ms with the columns shared out up to here, a
+// quarter more up to eight groups; in deep contact, sharing out always took 6.1 ms
+// against 5.1.
 constexpr int kSplitGroups = 4;
 // Points per thread in flight in the pass over the touch bits.
 constexpr int kAhead = 4;
@@ -581,7 +585,8 @@ struct Lists
     }
 };
 
-// The Jacobian of the listed points in contact, into kLists partial sums.
+// The Jacobian of the points in contact, in kForceRows lists, into as many
+// sums (kJacRows with touch bits).
 template <int MODE, bool SPARSE, int BD, bool TOUCH, int T>
 __device__ __forceinline__ void jacobian_pass(const GridView& g, const float* __restrict__ qx,
                                               const float* __restrict__ qw, const sdfo_body_state& sA,
@@ -589,9 +594,9 @@ __device__ __forceinline__ void jacobian_pass(const GridView& g, const float* __
                                               const sdfo_contact_params& prm, double narrow, const int* list,
                                               const int* lengths, double (*sums)[36])
 {
-    constexpr int kWarps = T / 32, kLists = TOUCH ? kRows : kWarps;
+    constexpr int kWarps = T / 32, kRows = TOUCH ? kJacRows : kWarps;
     const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
-    const Lists<kLists> lists(lengths);
+    const Lists<kForceRows> lists(lengths);
     auto add_column = [&](const double col[6], int row, int j) {
 #pragma unroll
         for (int r = 0; r < 6; ++r)
@@ -615,7 +620,7 @@ __device__ __forceinline__ void jacobian_pass(const GridView& g, const float* __
             double col[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
             PointState st;
             if (in_contact(e, at, st)) jacobian_column(st, sB, f, prm, k % 6, col);
-            add_column(col, k % kLists, k % 6);
+            add_column(col, k % kRows, k % 6);
         }
         return;
     }
@@ -629,7 +634,7 @@ __device__ __forceinline__ void jacobian_pass(const GridView& g, const float* __
         {
             double col[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
             if (mine) jacobian_column(st, sB, f, prm, j, col);
-            add_column(col, k % kLists, j);
+            add_column(col, k % kRows, j);
         }
     }
 }
@@ -662,25 +667,24 @@ __global__ void __launch_bounds__(T, MB)
               sdfo_contact_measure* __restrict__ meas, const uint32_t* __restrict__ bits)
 {
     constexpr int kWarps = T / 32;
-    constexpr int kLists = TOUCH ? kRows : kWarps, kPerList = kJacSpan / kLists;
-    constexpr int kOwn = kLists / kWarps; // lists and sums w, w + kWarps, .. are warp w's
+    constexpr int kPerList = kJacSpan / kWarps, kPerAct = kJacSpan / kForceRows;
+    constexpr int kRows = TOUCH ? kJacRows : kWarps; // sums of the Jacobian
     const int pose = blockIdx.x;
     __shared__ sdfo_body_state sA, sB;
-    __shared__ double red[kLists][6];
-    __shared__ double sjac[JAC ? kLists : 1][36];
+    __shared__ double red[kForceRows][6];
+    __shared__ double sjac[JAC ? kRows : 1][36];
     constexpr bool LIST = JAC || TOUCH;
     __shared__ int s_list[LIST ? kJacSpan : 1];
     __shared__ int s_act[TOUCH && JAC ? kJacSpan : 1];
-    __shared__ int s_acnt[kLists];
+    __shared__ int s_acnt[kForceRows];
     __shared__ Place32 s_touch;
-    __shared__ int s_wcnt[kLists];
+    __shared__ int s_wcnt[kWarps];
     __shared__ BroadShared s_broad;
     __shared__ MeasureShared<kWarps> s_meas;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     load_states(poses + pose, body_b, sA, sB);
     if (JAC)
-        for (int t = threadIdx.x; t < kLists * 36; t += T) (&sjac[0][0])[t] = 0.0;
-    if (TOUCH && threadIdx.x < kLists * 6) (&red[0][0])[threadIdx.x] = 0.0;
+        for (int t = threadIdx.x; t < kRows * 36; t += T) (&sjac[0][0])[t] = 0.0;
     __syncthreads();
     const PoseFrame f = pose_frame(sA, sB);
     Place32 tf;
@@ -725,7 +729,9 @@ __global__ void __launch_bounds__(T, MB)
     for (int s0 = 0; s0 < nq; s0 += LIST ? kJacSpan : nq)
     {
     const int s1 = LIST ? min(nq, s0 + kJacSpan) : nq;
-    int wcnt[kOwn] = {}; // listed points of the warp's lists (warp-uniform)
+    // this warp's list: the place of its half in the order of all (see kForceRows)
+    const int half = (warp % kForceRows) * (kWarps / kForceRows) + warp / kForceRows;
+    int wcnt = 0; // its points (warp-uniform)
     // appends the lanes' points to a list of which `count` are filled
     auto append = [&](int* list, int& count, bool listed, int i) {
         const unsigned m = __ballot_sync(0xffffffffu, listed);
@@ -736,14 +742,16 @@ __global__ void __launch_bounds__(T, MB)
     {
         // kAhead points per thread at a time: their loads, and then those of
         // their bits, are in flight together
-        for (int i0 = s0 + (int)threadIdx.x; i0 - (int)threadIdx.x < s1; i0 += kAhead * T)
+        constexpr int kStride = 32 * kForceRows;
+        const int base = s0 + 32 * (warp % kForceRows) + kJacSpan * kForceRows / kWarps * (warp / kForceRows) + lane;
+        for (int j = 0; j < kPerList / 32 && base - lane + j * kStride < s1; j += kAhead)
         {
             float x[kAhead][3];
             bool in[kAhead];
 #pragma unroll
             for (int u = 0; u < kAhead; ++u)
             {
-                const int i = i0 + u * T;
+                const int i = base + (j + u) * kStride;
                 in[u] = i < s1 && kept(i);
 #pragma unroll
                 for (int a = 0; a < 3; ++a) x[u][a] = in[u] ? __ldg(qx + 3 * i + a) : 0.f;
@@ -755,8 +763,7 @@ __global__ void __launch_bounds__(T, MB)
             for (int u = 0; u < kAhead; ++u)
             {
                 if (want_meas && in[u] && status[u] == kClear) ++seen.nvalid;
-                append(s_list + (warp + (u % kOwn) * kWarps) * kPerList, wcnt[u % kOwn], in[u] && status[u] == kMayTouch,
-                       i0 + u * T);
+                append(s_list + half * kPerList, wcnt, in[u] && status[u] == kMayTouch, base + (j + u) * kStride);
             }
         }
     }
@@ -776,29 +783,25 @@ __global__ void __launch_bounds__(T, MB)
                 act = status == 2 && want_force;
                 if (act) add_force(st, acc);
             }
-            if (LIST) append(s_list + warp * kPerList, wcnt[0], act, i);
+            if (LIST) append(s_list + warp * kPerList, wcnt, act, i);
         }
     }
     if (LIST)
     {
-        if (lane == 0)
-#pragma unroll
-            for (int o = 0; o < kOwn; ++o) s_wcnt[warp + o * kWarps] = wcnt[o];
+        if (lane == 0) s_wcnt[TOUCH ? half : warp] = wcnt;
         __syncthreads();
         if constexpr (TOUCH)
         {
-            const Lists<kLists> lists(s_wcnt);
+            const Lists<kWarps> lists(s_wcnt);
             if (lists.total == 0)
             {
                 __syncthreads();
                 continue;
             }
-#pragma unroll 1
-            for (int row = warp; row < kRows; row += kWarps) // warp-uniform
+            if (warp < kForceRows)
             {
                 int acnt = 0;
-                double sum[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-                for (int k = row; 32 * k < lists.total; k += kRows)
+                for (int k = warp; 32 * k < lists.total; k += kForceRows) // warp-uniform
                 {
                     const int e = 32 * k + lane, at = lists.place(e);
                     bool act = false;
@@ -812,20 +815,11 @@ __global__ void __launch_bounds__(T, MB)
                                                                                 want_meas, st, gap);
                         if (want_meas && status > 0) seen.point(cull, full, idx, gap);
                         act = status == 2 && want_force;
-                        if (act) add_force(st, sum);
+                        if (act) add_force(st, acc);
                     }
-                    if (JAC) append(s_act + row * kPerList, acnt, act, idx);
+                    if (JAC) append(s_act + warp * kPerAct, acnt, act, idx);
                 }
-                if (JAC && lane == 0) s_acnt[row] = acnt;
-                if (want_force && 32 * row < lists.total)
-                {
-#pragma unroll
-                    for (int q = 0; q < 6; ++q)
-                    {
-                        const double v = warp_sum(sum[q]);
-                        if (lane == 0) red[row][q] += v;
-                    }
-                }
+                if (JAC && lane == 0) s_acnt[warp] = acnt;
             }
             if (JAC) __syncthreads();
         }
@@ -851,7 +845,7 @@ __global__ void __launch_bounds__(T, MB)
                     seen.point(cull, full, i, gap);
             }
     }
-    if (!TOUCH && want_force)
+    if (want_force && warp < kForceRows)
     {
 #pragma unroll
         for (int q = 0; q < 6; ++q)
@@ -863,11 +857,11 @@ __global__ void __launch_bounds__(T, MB)
     __syncthreads();
     if (want_force && threadIdx.x < 6)
     {
-        ft[6 * (int64_t)pose + threadIdx.x] = row_sum<kLists>(&red[0][threadIdx.x], 6);
+        ft[6 * (int64_t)pose + threadIdx.x] = row_sum<kForceRows>(&red[0][threadIdx.x], 6);
     }
     if (JAC && jac != nullptr && threadIdx.x < 36)
     {
-        jac[36 * (int64_t)pose + threadIdx.x] = row_sum<kLists>(&sjac[0][threadIdx.x], 36);
+        jac[36 * (int64_t)pose + threadIdx.x] = row_sum<kRows>(&sjac[0][threadIdx.x], 36);
     }
     if (want_meas)
         write_measure<MODE, SPARSE, BD, T>(g, qx, sA, sB, f, cull, full, s_broad, s_meas, seen, meas + pose);
@@ -1019,9 +1013,10 @@ void launch4(const GridView& v, const ContactLaunch& c, const uint32_t* bits, cu
             launch5<MODE, SPARSE, BD, EXT, TOUCH, kFewThreads, 1, 1>(v, c, bits, s);
             return;
         }
-        // Trilinear Jacobians with touch bits gain by a third CTA where there are
-        // poses for it: 4,096 poses, a quarter in light contact, 321 us against
-        // 301; 149 poses in deep contact lose by it, 448 us against 514.
+        // Trilinear Jacobians with touch bits gain by a third CTA per SM where there
+        // are poses for it (4,096 poses, a quarter in light contact: 5 %), and lose
+        // by its spills where there are not (149 poses in deep contact: 448 us with
+        // two, 514 with three).
         if constexpr (MODE == SDFO_TRILINEAR)
             if (c.jac && c.np > 2 * current_sm_count())
             {
